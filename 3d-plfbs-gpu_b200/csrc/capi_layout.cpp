@@ -409,7 +409,7 @@ int build_compact_layout(plfbs_ctx* ctx) {
         TRY(pool_alloc(ctx, &p, 4 * (size_t)U));
         void* relax = nullptr;
         TRY(pool_alloc(ctx, &relax, 16 * (size_t)U));
-        plfbs::launch_record_sides(t[0], t[1], t[2], U, ctx->cfg.flavour,
+        plfbs::launch_record_sides(t[0], t[1], t[2], a.eq_cd, U, ctx->cfg.flavour,
                                    static_cast<int32_t*>(p), static_cast<double*>(relax),
                                    ctx->stream);
         a.frec_sides = static_cast<const int32_t*>(p);

@@ -22,52 +22,12 @@
 
 #include <cstdint>
 
+#include "flux_core.cuh"
 #include "ibm_spread.cuh"
 #include "plfbs_internal.hpp"
 
 namespace plfbs {
 namespace {
-
-struct __align__(32) d4 {
-  double x, y, z, w;
-};
-
-// Records of four doubles move as one 256-bit access (a whole 32-byte
-// sector per thread; every record array is 32-byte aligned): half the load
-// and store instructions of two 128-bit halves (step 0.541 -> 0.502 ms).
-// Read-only data: non-coherent load the compiler may schedule freely.
-__device__ __forceinline__ d4 ld4(const void* base, long long i) {
-  const double* p = reinterpret_cast<const double*>(base) + 4 * i;
-  d4 v;
-  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-      : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
-      : "l"(p));
-  return v;
-}
-// Coherent load, for data the same kernel also writes (kept in order).
-__device__ __forceinline__ d4 ld4rw(const void* base, long long i) {
-  const double* p = reinterpret_cast<const double*>(base) + 4 * i;
-  d4 v;
-  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
-               : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
-               : "l"(p)
-               : "memory");
-  return v;
-}
-__device__ __forceinline__ void st4(void* base, long long i, const d4& v) {
-  double* p = reinterpret_cast<double*>(base) + 4 * i;
-  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.x), "d"(v.y), "d"(v.z),
-               "d"(v.w)
-               : "memory");
-}
-
-// The same pointer, opaque to the compiler, so that a load through it is not
-// merged with an earlier load of the same address (a deliberate re-read).
-template <typename T>
-__device__ __forceinline__ const T* launder(const T* p) {
-  asm("mov.b64 %0, %0;" : "+l"(p));
-  return p;
-}
 
 // Whether the context has converged or diverged. One thread per block reads
 // the flag; every thread of the block must call this (it synchronises).
@@ -76,50 +36,6 @@ __device__ __forceinline__ bool halted(const KernelArgs& a) {
   if (threadIdx.x == 0) h = *(volatile const int*)&a.stats->halt;
   __syncthreads();
   return h != 0;
-}
-
-// Ghost state from its owner. FL = 0 (GPU kernels, update_unstructured_bcs
-// in LBFS.cu:1228-1301): bc1 holds the Dirichlet target, the raw value or for
-// the parabolic inlet (vel type 9) the profile 16 u (H/2+y)(H/2-y)(H/2+z)(H/2-z)/H^4
-// in x. FL = 1 (CPU Solver, Solution::update_unstructured_bcs,
-// Solution.cpp:759-833): rho 1 mirror, 2 copy, 6 and 7 the value; velocity 1
-// mirror, 2 copy, 6 the value, 8 (u, -v, w) of the owner.
-template <int FL>
-__device__ __forceinline__ d4 ghost_state(const d4& q, const d4& tgt, int types) {
-  const int rt = types & 0xff, vt = types >> 8;
-  d4 g;
-  if (FL == 1) {
-    g.w = rt == 1 ? tgt.w - (q.w - tgt.w) : (rt == 2 ? q.w : tgt.w);
-    if (vt == 1) {
-      g.x = tgt.x - (q.x - tgt.x);
-      g.y = tgt.y - (q.y - tgt.y);
-      g.z = tgt.z - (q.z - tgt.z);
-    } else if (vt == 2) {
-      g.x = q.x;
-      g.y = q.y;
-      g.z = q.z;
-    } else if (vt == 8) {
-      g.x = q.x;
-      g.y = -q.y;
-      g.z = q.z;
-    } else {
-      g.x = tgt.x;
-      g.y = tgt.y;
-      g.z = tgt.z;
-    }
-    return g;
-  }
-  g.w = (rt == 1) ? tgt.w - (q.w - tgt.w) : q.w;
-  if (vt == 2) {
-    g.x = q.x;
-    g.y = q.y;
-    g.z = q.z;
-  } else {
-    g.x = tgt.x - (q.x - tgt.x);
-    g.y = tgt.y - (q.y - tgt.y);
-    g.z = tgt.z - (q.z - tgt.z);
-  }
-  return g;
 }
 
 // ---------------------------------------------------------------------------
@@ -194,267 +110,6 @@ __global__ void __launch_bounds__(kBlock) k_gradient(const KernelArgs a) {
 // ---------------------------------------------------------------------------
 // flux
 // ---------------------------------------------------------------------------
-// Gradients as 12 doubles: rho, u, v, w, each (x, y, z).
-__device__ __forceinline__ void load_grad(const void* base, int c, double g[12]) {
-  const d4 a0 = ld4(base, 3LL * c), a1 = ld4(base, 3LL * c + 1), a2 = ld4(base, 3LL * c + 2);
-  g[0] = a0.x; g[1] = a0.y; g[2] = a0.z; g[3] = a0.w;
-  g[4] = a1.x; g[5] = a1.y; g[6] = a1.z; g[7] = a1.w;
-  g[8] = a2.x; g[9] = a2.y; g[10] = a2.z; g[11] = a2.w;
-}
-
-// Ghost gradient. FL = 0 (get_bc_gradients, LBFS.cu:1306-1416): Dirichlet
-// 2 (bc - q_owner) / |d| * d_hat from the raw boundary value (bc2 = (d_hat,
-// |d|)); Neumann the owner's gradient times (1 - |n|) componentwise (bc3).
-// FL = 1 (gradients::Get_LS_Gradients and get_ghost_grads,
-// gradients.cpp:395-506,592-648): Dirichlet (rho 1, velocity 1 and 8) along
-// the face normal (bc2 = (n, |d|)), Neumann times (1 - n) (bc3), types 6 zero,
-// rho 7 the owner's gradient.
-template <int FL>
-__device__ __forceinline__ void ghost_grad(const d4& q, const double go[12], const d4& bv,
-                                           const d4& dd, const d4& nm, int types,
-                                           double g[12]) {
-  const int rt = types & 0xff, vt = types >> 8;
-  const double dir[3] = {dd.x, dd.y, dd.z}, m[3] = {nm.x, nm.y, nm.z};
-  const double dq[4] = {2 * (bv.w - q.w), 2 * (bv.x - q.x), 2 * (bv.y - q.y), 2 * (bv.z - q.z)};
-  if constexpr (FL == 1) {
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-      const int t = f == 0 ? rt : vt;
-#pragma unroll
-      for (int c = 0; c < 3; c++)
-        g[3 * f + c] = (t == 1 || (f > 0 && t == 8)) ? dq[f] / dd.w * dir[c]
-                       : t == 2                      ? go[3 * f + c] * m[c]
-                       : t == 7                      ? go[3 * f + c]
-                                                     : 0.0;
-    }
-  } else {
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-      const bool dirichlet = (f == 0) ? (rt == 1) : (vt != 2);
-#pragma unroll
-      for (int c = 0; c < 3; c++)
-        g[3 * f + c] = dirichlet ? dq[f] / dd.w * dir[c] : go[3 * f + c] * m[c];
-    }
-  }
-}
-
-// A cell value at the face, q - t . g (t the offset from the face centroid
-// to the cell centroid), as three fused multiply-adds.
-__device__ __forceinline__ double reconstruct(double q, const double t[3], const double* g) {
-  return fma(-t[2], g[2], fma(-t[1], g[1], fma(-t[0], g[0], q)));
-}
-
-template <int EX, int EY, int EZ>
-__device__ __forceinline__ double edot(const double* g) {
-  // e . g for a lattice direction with components in {-1, 0, 1}
-  double s = 0.0;
-  if (EX) s = EX > 0 ? g[0] : -g[0];
-  if (EY) s = EY > 0 ? s + g[1] : s - g[1];
-  if (EZ) s = EZ > 0 ? s + g[2] : s - g[2];
-  return s;
-}
-
-// e . g of a gradient inside lattice_pair. The diagonal pairs (all of e's
-// components nonzero) come after the axis pairs and see each gradient as
-// (gx + gy, gx - gy, gz); every diagonal e . g is then one addition, and
-// rounds exactly as edot's (gx +- gy) +- gz.
-template <int EX, int EY, int EZ>
-__device__ __forceinline__ double gdot(const double* g) {
-  if (EX == 0 || EY == 0 || EZ == 0) return edot<EX, EY, EZ>(g);
-  static_assert(!(EX && EY && EZ) || EX == 1 || (EY == 1 && EZ == 1), "diagonal set");
-  if (EX == 1 && EY == 1) return EZ > 0 ? g[0] + g[2] : g[0] - g[2];
-  if (EX == 1) return g[1] + g[2];  // (1, -1, 1)
-  return g[2] - g[1];               // (-1, 1, 1)
-}
-
-// Branch of a lattice pair from s = e . n (see lattice_pair), as two bits.
-// FL = 1 (the CPU Solver, Solver.cpp:840-1274) has no dead band: s == 0 takes
-// both nodes from the owner side (3).
-template <int EX, int EY, int EZ, int FL>
-__device__ __forceinline__ unsigned pair_side(const double n[3], double d1) {
-  const double s = (EX ? (EX > 0 ? n[0] : -n[0]) : 0.0) + (EY ? (EY > 0 ? n[1] : -n[1]) : 0.0) +
-                   (EZ ? (EZ > 0 ? n[2] : -n[2]) : 0.0);
-  if (FL == 1) return s > 0.0 ? 1u : (s < 0.0 ? 2u : 3u);
-  return s > d1 ? 1u : (s < -d1 ? 2u : 0u);
-}
-
-// One opposite pair (k, k') of D3Q15 lattice nodes, e_k' = -e_k = -e, node k
-// at x_f - e dt_s (populate_lattice_macros, LBFS.cu:330-938). With s = e . n:
-// s > d1 takes node k from the owner side and k' from the neighbour side,
-// s < -d1 the reverse, otherwise both from the face average with averaged
-// gradients (the +-0.001 dt dead band, LBFS.cu:353-354). Their equilibria
-// (populate_feq, LBFS.cu:942-1038) are accumulated into the moments
-// rho_I, m = sum e f and P = sum e e^T f (xx, yy, zz, xy, xz, yz). A diagonal
-// pair adds the same f_k + f_k' to rho_I, P_xx, P_yy and P_zz: those pairs sum
-// it once into D, which the caller adds to the four.
-template <int EX, int EY, int EZ, int FL>
-__device__ __forceinline__ void lattice_pair(const double si[4], const double sn[4],
-                                             const double sc[4], const double g1[12],
-                                             const double g2[12], int side, double dt,
-                                             const double K[4], double& rhoI, double m[3],
-                                             double P[6], double& D) {
-  constexpr bool diag = EX != 0 && EY != 0 && EZ != 0;
-  // side (pair_side): 1 if s > d1, 2 if s < -d1, 0 in the dead band. Faces are
-  // sorted by their branch signature, so these branches are uniform across
-  // almost every warp; each computes only its own values.
-  double qa[4], qb[4];
-  if (side == 1) {
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-      qa[f] = fma(-gdot<EX, EY, EZ>(g1 + 3 * f), dt, si[f]);
-      qb[f] = fma(gdot<EX, EY, EZ>(g2 + 3 * f), dt, sn[f]);
-    }
-  } else if (side == 2) {
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-      qa[f] = fma(-gdot<EX, EY, EZ>(g2 + 3 * f), dt, sn[f]);
-      qb[f] = fma(gdot<EX, EY, EZ>(g1 + 3 * f), dt, si[f]);
-    }
-  } else if (FL == 1) {  // side 3: both nodes from the owner side
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-      const double e = gdot<EX, EY, EZ>(g1 + 3 * f);
-      qa[f] = fma(-e, dt, si[f]);
-      qb[f] = fma(e, dt, si[f]);
-    }
-  } else {
-    const double hdt = 0.5 * dt;  // e . (g1 + g2) / 2 dt
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-      const double e = gdot<EX, EY, EZ>(g1 + 3 * f) + gdot<EX, EY, EZ>(g2 + 3 * f);
-      qa[f] = fma(-e, hdt, sc[f]);
-      qb[f] = fma(e, hdt, sc[f]);
-    }
-  }
-  // w rho (1 + 3 e.u + 4.5 (e.u)^2 / gamma - 1.5 u^2 / gamma) as
-  // rho (w + 3w e.u + w c45 (e.u)^2 - w c15 u^2), K = (w, 3w, w c45, w c15)
-  // with c45 = 4.5 / gamma and c15 = 1.5 / gamma (kernel constants)
-  const double eua = edot<EX, EY, EZ>(qa + 1), eub = -edot<EX, EY, EZ>(qb + 1);
-  const double u2a = fma(qa[3], qa[3], fma(qa[2], qa[2], qa[1] * qa[1]));
-  const double u2b = fma(qb[3], qb[3], fma(qb[2], qb[2], qb[1] * qb[1]));
-  const double fa = qa[0] * fma(-K[3], u2a, fma(K[2] * eua, eua, fma(K[1], eua, K[0])));
-  const double fb = qb[0] * fma(-K[3], u2b, fma(K[2] * eub, eub, fma(K[1], eub, K[0])));
-  const double sum = fa + fb, dif = fa - fb;
-  // The axis pairs come first and each is the first to write its m and P
-  // component; (1, 1, 1) is the first diagonal pair: those writes assign.
-  constexpr bool first_diag = EX == 1 && EY == 1 && EZ == 1;
-  if (diag) {
-    if (EX) m[0] += EX > 0 ? dif : -dif;
-    if (EY) m[1] += EY > 0 ? dif : -dif;
-    if (EZ) m[2] += EZ > 0 ? dif : -dif;
-    const double p3 = (EX * EY > 0) ? sum : -sum, p4 = (EX * EZ > 0) ? sum : -sum,
-                 p5 = (EY * EZ > 0) ? sum : -sum;
-    if (first_diag) {
-      D = sum;
-      P[3] = p3;
-      P[4] = p4;
-      P[5] = p5;
-    } else {
-      D += sum;
-      P[3] += p3;
-      P[4] += p4;
-      P[5] += p5;
-    }
-  } else {
-    rhoI += sum;
-    if (EX) m[0] = EX > 0 ? dif : -dif;
-    if (EY) m[1] = EY > 0 ? dif : -dif;
-    if (EZ) m[2] = EZ > 0 ? dif : -dif;
-    if (EX) P[0] = sum;
-    if (EY) P[1] = sum;
-    if (EZ) P[2] = sum;
-  }
-}
-
-// Flux of one face (calc_face_flux, LBFS.cu:1592-1710 and
-// calculate_flux_at_interface, LBFS.cu:1042-1223), in closed form:
-//   rho_I = sum_k feq_k(lattice), m = sum_k e_k feq_k(lattice), u_I = m / rho_I
-//   f_k = feq_k(rho_I, u_I) - tau (feq_k(rho_I, u_I) - feq_k(lattice)),
-//   tau = 3 nu / (dt_s gamma)
-// whose moments are, exactly (D3Q15 equilibrium moments are isotropic):
-//   sum e f = m
-//   sum e e^T f = (1 - tau) (rho_I / 3 I + m m^T / (rho_I gamma)) + tau P_lattice
-// The face flux is (momentum, mass) = ((sum e e^T f) n, (sum e f) . n) A.
-// A boundary face (neighbour > n_cells in the reference) takes both sides from
-// the boundary value and all gradients from the ghost (LBFS.cu:356-401).
-// The face's moments and flux from its reconstructed values (si owner side,
-// sn neighbour side, sc their mean, each (rho, u, v, w)) and gradients g1, g2
-// (12 doubles each; transformed in place), n the unit normal and dt the
-// streaming dt.
-template <int FL, bool CR>
-__device__ __forceinline__ void face_flux_out(const KernelArgs& a, const int f, const int r,
-                                              const double n[3],
-                                              const double dt, const double si[4],
-                                              const double sn[4], const double sc[4],
-                                              double g1[12], double g2[12]) {
-  const double pg = a.pg;
-  // the seven branch decisions up front: n is not needed again until the end;
-  // with the compact layout they come precomputed per record (record_sides)
-  unsigned sides;
-  if (CR) {  // FP64 compact layouts always carry the record sides
-    sides = (unsigned)__ldg(a.frec_sides + r);
-  } else {
-    const double d1 = 0.001 * dt;
-    sides = pair_side<1, 0, 0, FL>(n, d1) | pair_side<0, 1, 0, FL>(n, d1) << 2 |
-            pair_side<0, 0, 1, FL>(n, d1) << 4 | pair_side<1, 1, 1, FL>(n, d1) << 6 |
-            pair_side<1, 1, -1, FL>(n, d1) << 8 | pair_side<1, -1, 1, FL>(n, d1) << 10 |
-            pair_side<-1, 1, 1, FL>(n, d1) << 12;
-  }
-  // centre node (k = 0): e = 0
-  const double u2c = fma(sc[3], sc[3], fma(sc[2], sc[2], sc[1] * sc[1]));
-  double rhoI = sc[0] * fma(-a.eq[0][3], u2c, a.eq[0][0]);
-  double m[3], P[6], D;  // first written by the pairs below (see lattice_pair)
-  lattice_pair<1, 0, 0, FL>(si, sn, sc, g1, g2, sides & 3, dt, a.eq[1], rhoI, m, P, D);
-  lattice_pair<0, 1, 0, FL>(si, sn, sc, g1, g2, sides >> 2 & 3, dt, a.eq[1], rhoI, m, P, D);
-  lattice_pair<0, 0, 1, FL>(si, sn, sc, g1, g2, sides >> 4 & 3, dt, a.eq[1], rhoI, m, P, D);
-#pragma unroll
-  for (int k = 0; k < 4; k++) {  // (gx, gy, gz) -> (gx + gy, gx - gy, gz), see gdot
-    const double s1 = g1[3 * k] + g1[3 * k + 1], r1 = g1[3 * k] - g1[3 * k + 1];
-    const double s2 = g2[3 * k] + g2[3 * k + 1], r2 = g2[3 * k] - g2[3 * k + 1];
-    g1[3 * k] = s1;
-    g1[3 * k + 1] = r1;
-    g2[3 * k] = s2;
-    g2[3 * k + 1] = r2;
-  }
-  lattice_pair<1, 1, 1, FL>(si, sn, sc, g1, g2, sides >> 6 & 3, dt, a.eq[2], rhoI, m, P, D);
-  lattice_pair<1, 1, -1, FL>(si, sn, sc, g1, g2, sides >> 8 & 3, dt, a.eq[2], rhoI, m, P, D);
-  lattice_pair<1, -1, 1, FL>(si, sn, sc, g1, g2, sides >> 10 & 3, dt, a.eq[2], rhoI, m, P, D);
-  lattice_pair<-1, 1, 1, FL>(si, sn, sc, g1, g2, sides >> 12 & 3, dt, a.eq[2], rhoI, m, P, D);
-  rhoI += D;
-  P[0] += D;
-  P[1] += D;
-  P[2] += D;
-
-  // n and A, and the relaxation factor tau = 3 nu / (dt_s gamma) as the
-  // pair ((1 - tau) A, tau A), are read again here (L1 hits; per record with
-  // the compact layout) rather than held in registers through the pairs.
-  const d4 g0 = ld4(launder(CR ? a.frec0 : a.face0), r);
-  const double nf[3] = {g0.x, g0.y, g0.z};
-  const double area = g0.w;
-  double omA, tA;
-  if (CR) {
-    const double2 w = __ldg(reinterpret_cast<const double2*>(a.frec_relax) + r);
-    omA = w.x;
-    tA = w.y;
-  } else {
-    const double tau = __ldg(static_cast<const double*>(launder(a.face2)) + 4LL * r + 3);
-    omA = (1.0 - tau) * area;
-    tA = tau * area;
-  }
-  const double mn = m[0] * nf[0] + m[1] * nf[1] + m[2] * nf[2];
-  const double Pn[3] = {P[0] * nf[0] + P[3] * nf[1] + P[4] * nf[2],
-                        P[3] * nf[0] + P[1] * nf[1] + P[5] * nf[2],
-                        P[4] * nf[0] + P[5] * nf[1] + P[2] * nf[2]};
-  const double p3 = rhoI * (1.0 / 3.0);
-  const double mnr = mn / rhoI * pg;
-  d4 out;
-  out.x = fma(omA, fma(m[0], mnr, p3 * nf[0]), tA * Pn[0]);
-  out.y = fma(omA, fma(m[1], mnr, p3 * nf[1]), tA * Pn[1]);
-  out.z = fma(omA, fma(m[2], mnr, p3 * nf[2]), tA * Pn[2]);
-  out.w = mn * area;
-  st4(a.flux, f, out);
-}
-
 __device__ __forceinline__ int2 face_ids(const KernelArgs& a, long long f) {
   return __ldg(reinterpret_cast<const int2*>(a.face_ids) + f);
 }
@@ -463,67 +118,27 @@ __device__ __forceinline__ int2 face_ids(const KernelArgs& a, long long f) {
 template <int FL, bool CR>
 __device__ __forceinline__ void flux_face(const KernelArgs& a, const int f, const int2 ids,
                                           const int rec) {
-  const d4 f0 = CR ? ld4(a.frec0, rec) : ld4(a.face0, f);
-  const d4 f1 = CR ? ld4(a.frec1, rec) : ld4(a.face1, f);
-  const d4 f2 = CR ? ld4(a.frec2, rec) : ld4(a.face2, f);
+  const int r = CR ? rec : f;
+  const d4 f0 = ld4(CR ? a.frec0 : a.face0, r), f1 = ld4(CR ? a.frec1 : a.face1, r),
+           f2 = ld4(CR ? a.frec2 : a.face2, r);
   const int o = ids.x, nb = ids.y;
-  const double n[3] = {f0.x, f0.y, f0.z};
   const double dt = f1.x;
   const double t1[3] = {f1.y, f1.z, f1.w}, t2[3] = {f2.x, f2.y, f2.z};
-
   const d4 qo = ld4(a.state, o);
   double g1[12], g2[12], si[4], sn[4], sc[4];
   load_grad(a.grad, o, g1);
-  const double qov[4] = {qo.w, qo.x, qo.y, qo.z};
-  bool interior = true;
-  d4 qn;
   if (nb < a.C) {
-    qn = ld4(a.state, nb);
+    const d4 qn = ld4(a.state, nb);
     load_grad(a.grad, nb, g2);
+    interior_sides(t1, t2, qo, qn, g1, g2, si, sn, sc);
   } else {
-    const int b = nb - a.C;
-    const d4 bv = ld4(a.bc0, b), tgt = ld4(a.bc1, b), dd = ld4(a.bc2, b), nm = ld4(a.bc3, b);
-    const int types = (int)nm.w;
-    ghost_grad<FL>(qo, g1, bv, dd, nm, types, g2);
-    if (b == a.quirk_b) {
-      // The reference tests neighbour > n_cells (LBFS.cu:356), so its first
-      // ghost (index n_cells) goes through the interior branch with the ghost
-      // state and gradient as the neighbour's.
-      qn = ghost_state<FL>(qo, tgt, types);
-    } else {
-      interior = false;
-      const int rt = types & 0xff, vt = types >> 8;
-      const double bvv[4] = {bv.w, bv.x, bv.y, bv.z};
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        // FL = 1 (populate_lattice_macros, Solver.cpp:862-904): rho 1 and
-        // velocity 1 the value, velocity 8 (u, 0, w) of the owner, otherwise
-        // extrapolated with the ghost gradient
-        const bool dirichlet = (k == 0) ? (rt == 1) : (FL == 1 ? vt == 1 : vt != 2);
-        const double ext = reconstruct(qov[k], t1, g2 + 3 * k);
-        sc[k] = dirichlet ? bvv[k] : (FL == 1 && k > 0 && vt == 8) ? (k == 2 ? 0.0 : qov[k]) : ext;
-        si[k] = sc[k];
-        sn[k] = sc[k];
-      }
-      // FL = 0: the ghost gradient on both sides (LBFS.cu:398-401); FL = 1
-      // keeps the owner's on the owner side
-      if (FL == 0) {
-#pragma unroll
-        for (int k = 0; k < 12; k++) g1[k] = g2[k];
-      }
-    }
+    boundary_sides<FL>(a, nb - a.C, t1, t2, qo, g1, g2, si, sn, sc);
   }
-  if (interior) {
-    const double qnv[4] = {qn.w, qn.x, qn.y, qn.z};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      si[k] = reconstruct(qov[k], t1, g1 + 3 * k);
-      sn[k] = reconstruct(qnv[k], t2, g2 + 3 * k);
-      sc[k] = (si[k] + sn[k]) * 0.5;
-    }
-  }
-
-  face_flux_out<FL, CR>(a, f, CR ? rec : f, n, dt, si, sn, sc, g1, g2);
+  // the branch decisions: per record with the compact layout (FP64 compact
+  // layouts always carry them)
+  const double n[3] = {f0.x, f0.y, f0.z};
+  const unsigned sides = CR ? (unsigned)__ldg(a.frec_sides + r) : face_sides<FL>(n, dt);
+  st4(a.flux, f, face_flux<FL, CR>(a, r, sides, dt, si, sn, sc, g1, g2));
 }
 
 // Persistent over the faces [f_begin, f_end) (grid stride): the
@@ -558,7 +173,7 @@ __global__ void __launch_bounds__(kFluxBlock, 4) k_flux(const KernelArgs a, int 
 // flux, TMA-staged (internal faces): a producer warp gathers each tile's cell
 // rows into shared memory with tile::gather4 bulk tensor copies while four
 // consumer warps compute the previous tile. The consumers never wait on a
-// global gather; the arithmetic per face is face_flux_out's.
+// global gather; the arithmetic per face is face_flux's.
 // ---------------------------------------------------------------------------
 constexpr int kTmaFaces = 128;  // faces per tile, one per consumer thread
 constexpr int kTmaStages = 2;
@@ -681,8 +296,8 @@ __global__ void __launch_bounds__(kTmaThreads, 3)
     const double* sn_ = reinterpret_cast<const double*>(st + kTmaSn) + 4 * c;
     const double* go = reinterpret_cast<const double*>(st + kTmaGo) + 12 * c;
     const double* gn = reinterpret_cast<const double*>(st + kTmaGn) + 12 * c;
-    // state rows are (u, v, w, rho)
-    const double qov[4] = {so[3], so[0], so[1], so[2]}, qnv[4] = {sn_[3], sn_[0], sn_[1], sn_[2]};
+    // state rows are (u, v, w, rho), read before the stage is handed back
+    const d4 qo{so[0], so[1], so[2], so[3]}, qn{sn_[0], sn_[1], sn_[2], sn_[3]};
     double g1[12], g2[12];
 #pragma unroll
     for (int i = 0; i < 12; i++) {
@@ -696,13 +311,8 @@ __global__ void __launch_bounds__(kTmaThreads, 3)
     const double dt = f1.x;
     const double t1[3] = {f1.y, f1.z, f1.w}, t2[3] = {f2.x, f2.y, f2.z};
     double si[4], sn[4], sc[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      si[q] = reconstruct(qov[q], t1, g1 + 3 * q);
-      sn[q] = reconstruct(qnv[q], t2, g2 + 3 * q);
-      sc[q] = (si[q] + sn[q]) * 0.5;
-    }
-    face_flux_out<0, false>(a, f, f, n, dt, si, sn, sc, g1, g2);
+    interior_sides(t1, t2, qo, qn, g1, g2, si, sn, sc);
+    st4(a.flux, f, face_flux<0, false>(a, f, face_sides<0>(n, dt), dt, si, sn, sc, g1, g2));
   }
 }
 
@@ -1073,35 +683,30 @@ __global__ void __launch_bounds__(kWallBlock) k_wall_forces(const KernelArgs a, 
 inline int blocks_for(long long n, int bs) { return (int)((n + bs - 1) / bs); }
 
 // The seven branch decisions of each unique face record of the compact
-// layout, as face_flux_out computes them.
+// layout and the area factors face_flux forms per face without it.
 template <int FL>
-__global__ void k_record_sides(const void* frec0, const void* frec1, const void* frec2, int n,
-                               int32_t* out, double2* relax) {
+__global__ void k_record_sides(const void* frec0, const void* frec1, const void* frec2, double cd,
+                               int n, int32_t* out, double2* relax) {
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     const d4 f0 = ld4(frec0, r), f1 = ld4(frec1, r), f2 = ld4(frec2, r);
-    // the pair face_flux_out forms per face without the compact layout
-    relax[r] = make_double2((1.0 - f2.w) * f0.w, f2.w * f0.w);
+    const double cA = __dmul_rn(f0.w, cd);
+    relax[r] = make_double2(__dmul_rn(__dadd_rn(1.0, -f2.w), cA), __dmul_rn(f2.w, cA));
     const double nv[3] = {f0.x, f0.y, f0.z};
-    const double d1 = 0.001 * f1.x;
-    out[r] = (int32_t)(pair_side<1, 0, 0, FL>(nv, d1) | pair_side<0, 1, 0, FL>(nv, d1) << 2 |
-                       pair_side<0, 0, 1, FL>(nv, d1) << 4 | pair_side<1, 1, 1, FL>(nv, d1) << 6 |
-                       pair_side<1, 1, -1, FL>(nv, d1) << 8 |
-                       pair_side<1, -1, 1, FL>(nv, d1) << 10 |
-                       pair_side<-1, 1, 1, FL>(nv, d1) << 12);
+    out[r] = (int32_t)face_sides<FL>(nv, f1.x);
   }
 }
 
 }  // namespace
 
-void launch_record_sides(const void* frec0, const void* frec1, const void* frec2, int n,
+void launch_record_sides(const void* frec0, const void* frec1, const void* frec2, double cd, int n,
                          int flavour, int32_t* out, double* relax, cudaStream_t s) {
   if (n <= 0) return;
   const int nb = (int)blocks_for(n, kBlock);
   double2* rl = reinterpret_cast<double2*>(relax);
   if (flavour == PLFBS_FLAVOUR_CPU_SOLVER)
-    k_record_sides<1><<<nb, kBlock, 0, s>>>(frec0, frec1, frec2, n, out, rl);
+    k_record_sides<1><<<nb, kBlock, 0, s>>>(frec0, frec1, frec2, cd, n, out, rl);
   else
-    k_record_sides<0><<<nb, kBlock, 0, s>>>(frec0, frec1, frec2, n, out, rl);
+    k_record_sides<0><<<nb, kBlock, 0, s>>>(frec0, frec1, frec2, cd, n, out, rl);
 }
 
 void launch_gradient(const KernelArgs& a, int precision, cudaStream_t s) {
