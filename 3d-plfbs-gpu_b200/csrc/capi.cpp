@@ -933,7 +933,7 @@ int plfbs_save_checkpoint(plfbs_ctx* ctx, void* buf, int64_t bytes) {
     e = cudaMemcpyAsync(out, stage, rec * (size_t)T, cudaMemcpyDeviceToHost, ctx->stream);
   out += rec * (size_t)T;
   if (e == cudaSuccess) {
-    plfbs::launch_records(ctx->perm, L.C, (int)rec, ctx->args.t1, stage, true, ctx->stream);
+    plfbs::launch_records(ctx->perm, L.C, (int)rec, ctx->args.t0, stage, true, ctx->stream);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess)
@@ -973,8 +973,8 @@ int plfbs_load_checkpoint(plfbs_ctx* ctx, const void* buf, int64_t bytes) {
   const size_t rec = ctx->cfg.precision == PLFBS_FP32_DEVIATION ? 16 : 32;
   const int64_t T = (int64_t)L.C + L.B;
   const char* in = static_cast<const char*>(buf) + sizeof h;
-  // scattered from the caller's order on the device; at a step boundary t0
-  // equals t1
+  // scattered from the caller's order on the device; at a step boundary the
+  // accumulator is t0
   void* stage = nullptr;
   TRY(scratch_alloc(ctx, &stage, rec * (size_t)T));
   cudaError_t e = cudaMemcpyAsync(stage, in, rec * (size_t)T, cudaMemcpyHostToDevice, ctx->stream);
@@ -986,12 +986,9 @@ int plfbs_load_checkpoint(plfbs_ctx* ctx, const void* buf, int64_t bytes) {
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(stage, in, rec * (size_t)L.C, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess) {
-    plfbs::launch_records(ctx->perm, L.C, (int)rec, stage, ctx->args.t1, false, ctx->stream);
+    plfbs::launch_records(ctx->perm, L.C, (int)rec, stage, ctx->args.t0, false, ctx->stream);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(ctx->args.t0, ctx->args.t1, rec * (size_t)L.C, cudaMemcpyDeviceToDevice,
-                        ctx->stream);
   scratch_free(ctx, stage);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess)

@@ -468,5 +468,27 @@ __device__ __forceinline__ d4 face_flux(const KernelArgs& a, const int r, const 
   return flux_of_moments(a.pg, R, m, P, n, cA, omA, tA);
 }
 
+// One cell's RK stage (time_integration, LBFS.cu:1457-1521) from its residual R
+// (u, v, w, rho): the stage state q and the accumulator. t0 is the step's
+// start, t1 the running accumulator; at a step boundary they are equal (the
+// next step starts from the accumulator, Solver_gpu.cu:671), so stage 0 takes
+// t0 for both and stage 3, whose state is the accumulator's, does not need t0.
+template <int RK>
+__device__ __forceinline__ void rk_stage(const double dt, const d4& t0, const d4& t1,
+                                         const double R[4], d4& q, d4& acc) {
+  constexpr double alpha = (RK == 0 || RK == 3) ? 1.0 : 0.5;
+  constexpr double beta = (RK == 0 || RK == 3) ? (1.0 / 6.0) : (1.0 / 3.0);
+  const double bdt = __dmul_rn(dt, beta);
+  const d4& b = RK == 0 ? t0 : t1;
+  acc = d4{fma(R[0], bdt, b.x), fma(R[1], bdt, b.y), fma(R[2], bdt, b.z), fma(R[3], bdt, b.w)};
+  if (RK == 3) {
+    q = d4{__ddiv_rn(acc.x, acc.w), __ddiv_rn(acc.y, acc.w), __ddiv_rn(acc.z, acc.w), acc.w};
+  } else {
+    const double adt = __dmul_rn(dt, alpha), f = fma(R[3], adt, t0.w);
+    q = d4{__ddiv_rn(fma(R[0], adt, t0.x), f), __ddiv_rn(fma(R[1], adt, t0.y), f),
+           __ddiv_rn(fma(R[2], adt, t0.z), f), f};
+  }
+}
+
 }  // namespace
 }  // namespace plfbs

@@ -330,15 +330,16 @@ template <int RK, int K2MAX>
 __global__ void __launch_bounds__(kBlock) k_update(const KernelArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (halted(a)) return;  // uniform across the launch
-  constexpr double alpha = (RK == 0 || RK == 3) ? 1.0 : 0.5;
-  constexpr double beta = (RK == 0 || RK == 3) ? (1.0 / 6.0) : (1.0 / 3.0);
   double sq[4] = {0.0, 0.0, 0.0, 0.0};
   bool bad = false;
   if (i < a.C) {
     // The RK accumulators are loaded first, with the gather, so no store of
-    // the stage can come between them and the flux loads.
-    const d4 t0 = ld4rw(a.t0, i);
-    d4 t1 = ld4rw(a.t1, i);
+    // the stage can come between them and the flux loads. A stage moves only
+    // those it needs (rk_stage): the step's start t0 in stages 0-2, the
+    // accumulator t1 read in 1-3 and written in 0-2, the finished one to t0.
+    d4 t0{}, t1{};
+    if (RK != 3) t0 = ld4rw(a.t0, i);
+    if (RK != 0) t1 = ld4rw(a.t1, i);
     double r[4] = {0.0, 0.0, 0.0, 0.0};
     if (K2MAX > 0) {
       int e[K2MAX > 0 ? K2MAX : 1];
@@ -379,28 +380,16 @@ __global__ void __launch_bounds__(kBlock) k_update(const KernelArgs a) {
       R[0] += a.pressure_gradient;
     }
     if (a.res_debug) st4(a.res_debug, i, d4{R[0], R[1], R[2], R[3]});
-    const double dt = a.dt;
-    double f1 = t0.w + R[3] * dt * alpha;
-    double f2 = t0.x + R[0] * dt * alpha;
-    double f3 = t0.y + R[1] * dt * alpha;
-    double f4 = t0.z + R[2] * dt * alpha;
-    t1.w = t1.w + dt * beta * R[3];
-    t1.x = t1.x + dt * beta * R[0];
-    t1.y = t1.y + dt * beta * R[1];
-    t1.z = t1.z + dt * beta * R[2];
-    d4 q;
+    d4 q, acc;
+    rk_stage<RK>(a.dt, t0, t1, R, q, acc);
     if (RK == 3) {
-      q = d4{t1.x / t1.w, t1.y / t1.w, t1.z / t1.w, t1.w};
-      st4(a.t0, i, t1);  // the next step starts from t1 (Solver_gpu.cu:671)
       sq[0] = R[3] * R[3];
       sq[1] = R[0] * R[0];
       sq[2] = R[1] * R[1];
       sq[3] = R[2] * R[2];
-      bad = !(t1.w <= 1000.0);  // the CPU solver's divergence test, Solver.cpp:448-493
-    } else {
-      q = d4{f2 / f1, f3 / f1, f4 / f1, f1};
+      bad = !(acc.w <= 1000.0);  // the CPU solver's divergence test, Solver.cpp:448-493
     }
-    st4(a.t1, i, t1);
+    st4(RK == 3 ? a.t0 : a.t1, i, acc);
     st4(a.state, i, q);
     // The last reader of this step's force resets it for the IBM. The stores
     // come after every load of the stage: placed before the t0/t1 loads they
@@ -491,8 +480,8 @@ __global__ void __launch_bounds__(kFinishBlock) k_finish(const KernelArgs a) {
   }
 }
 
-// Seeds the RK accumulator from the state (Solver_gpu.cu:664): t0 = t1 = q.
-// The reference seeds the velocity state although the stages treat t0/t1 as
+// Seeds the RK accumulator from the state (Solver_gpu.cu:664): t0 = q (t1 is
+// written by the first stage before it is read). The reference seeds the velocity state although the stages treat t0/t1 as
 // (rho u, rho v, rho w, rho); with conserved = true (warm starts, no reference
 // counterpart) the accumulators get the conserved variables instead.
 template <bool CONSERVED>
@@ -502,7 +491,6 @@ __global__ void k_seed(const KernelArgs a) {
   d4 q = ld4(a.state, i);
   if (CONSERVED) q = d4{q.w * q.x, q.w * q.y, q.w * q.z, q.w};
   st4(a.t0, i, q);
-  st4(a.t1, i, q);
 }
 
 // ---------------------------------------------------------------------------

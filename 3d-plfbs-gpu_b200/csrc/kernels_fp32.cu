@@ -372,6 +372,26 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// One cell's RK stage in deviation units (as rk_stage in flux_core.cuh).
+template <int RK>
+__device__ __forceinline__ void rk_stage32(const float dt, const float rho0, const f4& t0,
+                                           const f4& t1, const float R[4], f4& q, f4& acc) {
+  constexpr float alpha = (RK == 0 || RK == 3) ? 1.0f : 0.5f;
+  constexpr float beta = (RK == 0 || RK == 3) ? (1.0f / 6.0f) : (1.0f / 3.0f);
+  const float bdt = __fmul_rn(dt, beta);
+  const f4& b = RK == 0 ? t0 : t1;
+  acc = f4{fmaf(R[0], bdt, b.x), fmaf(R[1], bdt, b.y), fmaf(R[2], bdt, b.z),
+           fmaf(R[3], bdt, b.w)};
+  f4 f = acc;
+  if (RK != 3) {
+    const float adt = __fmul_rn(dt, alpha);
+    f = f4{fmaf(R[0], adt, t0.x), fmaf(R[1], adt, t0.y), fmaf(R[2], adt, t0.z),
+           fmaf(R[3], adt, t0.w)};
+  }
+  const float rho = __fadd_rn(rho0, f.w);
+  q = f4{__fdiv_rn(f.x, rho), __fdiv_rn(f.y, rho), __fdiv_rn(f.z, rho), f.w};
+}
+
 // Gather + body force + RK stage in deviation units; the last stage reduces
 // the squared residuals in FP64 (momentum residuals are already divided by U,
 // so inv_ref_mom is 1 / rho_ref here).
@@ -379,15 +399,15 @@ template <int RK, int K2MAX>
 __global__ void __launch_bounds__(kBlock) k_update32(const KernelArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (halted(a)) return;
-  constexpr float alpha = (RK == 0 || RK == 3) ? 1.0f : 0.5f;
-  constexpr float beta = (RK == 0 || RK == 3) ? (1.0f / 6.0f) : (1.0f / 3.0f);
   double sq[4] = {0.0, 0.0, 0.0, 0.0};
   bool bad = false;
   if (i < a.C) {
-    // The RK accumulators are loaded first, with the gather, so no store of
-    // the stage can come between them and the flux loads.
-    const f4 t0 = ldf_rw(a.t0, i);
-    f4 t1 = ldf_rw(a.t1, i);
+    // The RK accumulators a stage needs (as k_update), loaded first, with the
+    // gather, so no store of the stage can come between them and the flux
+    // loads.
+    f4 t0{}, t1{};
+    if (RK != 3) t0 = ldf_rw(a.t0, i);
+    if (RK != 0) t1 = ldf_rw(a.t1, i);
     float r[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     int e[K2MAX];
 #pragma unroll
@@ -416,30 +436,16 @@ __global__ void __launch_bounds__(kBlock) k_update32(const KernelArgs a) {
       R[0] += pgU;
     }
     if (a.res_debug) stf(a.res_debug, i, f4{R[0], R[1], R[2], R[3]});
-    const float dt = (float)a.dt;
-    const float f1 = t0.w + R[3] * dt * alpha;
-    const float f2 = t0.x + R[0] * dt * alpha;
-    const float f3 = t0.y + R[1] * dt * alpha;
-    const float f4v = t0.z + R[2] * dt * alpha;
-    t1.w = t1.w + dt * beta * R[3];
-    t1.x = t1.x + dt * beta * R[0];
-    t1.y = t1.y + dt * beta * R[1];
-    t1.z = t1.z + dt * beta * R[2];
-    f4 q;
+    f4 q, acc;
+    rk_stage32<RK>((float)a.dt, a.rho0f, t0, t1, R, q, acc);
     if (RK == 3) {
-      const float rho = a.rho0f + t1.w;
-      q = f4{t1.x / rho, t1.y / rho, t1.z / rho, t1.w};
-      stf(a.t0, i, t1);
       sq[0] = (double)R[3] * R[3];
       sq[1] = (double)R[0] * R[0];
       sq[2] = (double)R[1] * R[1];
       sq[3] = (double)R[2] * R[2];
-      bad = !(rho <= 1000.0f);
-    } else {
-      const float rho = a.rho0f + f1;
-      q = f4{f2 / rho, f3 / rho, f4v / rho, f1};
+      bad = !(a.rho0f + acc.w <= 1000.0f);
     }
-    stf(a.t1, i, t1);
+    stf(RK == 3 ? a.t0 : a.t1, i, acc);
     stf(a.state, i, q);
     if (RK == 3 && a.fforce_x) {  // after every load of the stage (see k_update)
       a.fforce_x[i] = pgU;
@@ -539,7 +545,6 @@ __global__ void k_seed32(const KernelArgs a) {
     q = f4{rho * q.x, rho * q.y, rho * q.z, q.w};
   }
   stf(a.t0, i, q);
-  stf(a.t1, i, q);
 }
 
 // IBM with FP64 node positions and forces; velocities interpolated from the
