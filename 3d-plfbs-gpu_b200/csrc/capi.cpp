@@ -573,6 +573,13 @@ int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh, const plf
   a.inv_ref_mom = fp32 ? 1.0 / cfg->ref_rho : 1.0 / (cfg->ref_rho * cfg->max_velocity);
   a.rho0 = cfg->ref_rho;
   a.uref = cfg->max_velocity;
+  {
+    const double c = 1.5 * a.uref * a.uref * a.pg;
+    a.eq32_k0 = (float)(1.0 / c);
+    a.eq32_k1 = (float)(2.0 * cfg->gamma / a.uref);
+    a.eq32_cd = (float)(c / 72.0);
+    a.eq32_pgcd = (float)(c / 72.0 * a.pg);
+  }
   a.rho0f = (float)cfg->ref_rho;
   a.inv_uref_f = (float)(1.0 / cfg->max_velocity);
   for (int c = 0; c < 3; c++) a.origin[c] = cfg->origin[c];

@@ -19,27 +19,12 @@
 
 #include <cstdint>
 
+#include "flux_core32.cuh"
 #include "ibm_spread.cuh"
 #include "plfbs_internal.hpp"
 
 namespace plfbs {
 namespace {
-
-struct __align__(16) f4 {
-  float x, y, z, w;
-};
-
-__device__ __forceinline__ f4 ldf(const void* base, long long i) {
-  const float4 v = __ldg(reinterpret_cast<const float4*>(base) + i);
-  return f4{v.x, v.y, v.z, v.w};
-}
-__device__ __forceinline__ f4 ldf_rw(const void* base, long long i) {
-  const float4 v = reinterpret_cast<const float4*>(base)[i];
-  return f4{v.x, v.y, v.z, v.w};
-}
-__device__ __forceinline__ void stf(void* base, long long i, const f4& v) {
-  reinterpret_cast<float4*>(base)[i] = make_float4(v.x, v.y, v.z, v.w);
-}
 
 // Whether the context has converged or diverged. One thread per block reads
 // the flag; every thread of the block must call this (it synchronises).
@@ -48,23 +33,6 @@ __device__ __forceinline__ bool halted(const KernelArgs& a) {
   if (threadIdx.x == 0) h = *(volatile const int*)&a.stats->halt;
   __syncthreads();
   return h != 0;
-}
-
-// Ghost state in deviation units (the same affine rules as the FP64 path).
-__device__ __forceinline__ f4 ghost_state32(const f4& q, const f4& tgt, int types) {
-  const int rt = types & 0xff, vt = types >> 8;
-  f4 g;
-  g.w = (rt == 1) ? tgt.w - (q.w - tgt.w) : q.w;
-  if (vt == 2) {
-    g.x = q.x;
-    g.y = q.y;
-    g.z = q.z;
-  } else {
-    g.x = tgt.x - (q.x - tgt.x);
-    g.y = tgt.y - (q.y - tgt.y);
-    g.z = tgt.z - (q.z - tgt.z);
-  }
-  return g;
 }
 
 // Gradient layout: 3 x float4 per cell: (rx ry rz ux)(uy uz vx vy)(vz wx wy wz).
@@ -126,114 +94,7 @@ __global__ void __launch_bounds__(kBlock) k_gradient32(const KernelArgs a) {
   stf(a.grad, 3LL * i + 2, f4{g[8], g[9], g[10], g[11]});
 }
 
-__device__ __forceinline__ void load_grad32(const void* base, int c, float g[12]) {
-  const f4 a0 = ldf(base, 3LL * c), a1 = ldf(base, 3LL * c + 1), a2 = ldf(base, 3LL * c + 2);
-  g[0] = a0.x; g[1] = a0.y; g[2] = a0.z; g[3] = a0.w;
-  g[4] = a1.x; g[5] = a1.y; g[6] = a1.z; g[7] = a1.w;
-  g[8] = a2.x; g[9] = a2.y; g[10] = a2.z; g[11] = a2.w;
-}
-
-__device__ __forceinline__ void ghost_grad32(const f4& q, const float go[12], const f4& bv,
-                                             const f4& dd, const f4& nm, int types, float g[12]) {
-  const int rt = types & 0xff, vt = types >> 8;
-  const float dir[3] = {dd.x, dd.y, dd.z}, m[3] = {nm.x, nm.y, nm.z};
-  const float dq[4] = {2.0f * (bv.w - q.w), 2.0f * (bv.x - q.x), 2.0f * (bv.y - q.y),
-                       2.0f * (bv.z - q.z)};
-#pragma unroll
-  for (int f = 0; f < 4; f++) {
-    const bool dirichlet = (f == 0) ? (rt == 1) : (vt != 2);
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-      g[3 * f + c] = dirichlet ? dq[f] / dd.w * dir[c] : go[3 * f + c] * m[c];
-  }
-}
-
-template <int EX, int EY, int EZ>
-__device__ __forceinline__ float edotf(const float* g) {
-  float s = 0.0f;
-  if (EX) s = EX > 0 ? g[0] : -g[0];
-  if (EY) s = EY > 0 ? s + g[1] : s - g[1];
-  if (EZ) s = EZ > 0 ? s + g[2] : s - g[2];
-  return s;
-}
-
-// e . g of a gradient; diagonal pairs see (gx + gy, gx - gy, gz) (as gdot in
-// kernels.cu).
-template <int EX, int EY, int EZ>
-__device__ __forceinline__ float gdotf(const float* g) {
-  if (EX == 0 || EY == 0 || EZ == 0) return edotf<EX, EY, EZ>(g);
-  if (EX == 1 && EY == 1) return EZ > 0 ? g[0] + g[2] : g[0] - g[2];
-  if (EX == 1) return g[1] + g[2];  // (1, -1, 1)
-  return g[2] - g[1];               // (-1, 1, 1)
-}
-
-// Consts shared by the lattice pairs of one face.
-struct PairConst {
-  float d1, dt, hdt;
-  float rho0, U, c45u, c15u;  // c45u = 4.5 U / gamma, c15u = 1.5 U / gamma
-  float u3, c45uu, c15uu;     // 3 U, U c45u, U c15u
-};
-
-// Deviation part of the equilibrium at one node: w [drho + rho U phi].
-__device__ __forceinline__ float feq_dev(const PairConst& k, float wgt, const float q[4],
-                                         float eu) {
-  const float u2 = fmaf(q[3], q[3], fmaf(q[2], q[2], q[1] * q[1]));
-  // U phi = U (3 eu + c45u eu^2 - c15u u2), with U folded into the constants
-  const float uphi = fmaf(eu, fmaf(k.c45uu, eu, k.u3), -k.c15uu * u2);
-  return wgt * fmaf(k.rho0 + q[0], uphi, q[0]);
-}
-
-template <int EX, int EY, int EZ>
-__device__ __forceinline__ void lattice_pair32(const float si[4], const float sn[4],
-                                               const float sc[4], const float g1[12],
-                                               const float g2[12], const float n[3],
-                                               const PairConst& k, float wgt, float& drhoI,
-                                               float m[3], float P[6], float& D) {
-  constexpr bool diag = EX != 0 && EY != 0 && EZ != 0;
-  const float s = (EX ? (EX > 0 ? n[0] : -n[0]) : 0.0f) + (EY ? (EY > 0 ? n[1] : -n[1]) : 0.0f) +
-                  (EZ ? (EZ > 0 ? n[2] : -n[2]) : 0.0f);
-  float qa[4], qb[4];
-  if (s > k.d1) {
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-      qa[f] = fmaf(-gdotf<EX, EY, EZ>(g1 + 3 * f), k.dt, si[f]);
-      qb[f] = fmaf(gdotf<EX, EY, EZ>(g2 + 3 * f), k.dt, sn[f]);
-    }
-  } else if (s < -k.d1) {
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-      qa[f] = fmaf(-gdotf<EX, EY, EZ>(g2 + 3 * f), k.dt, sn[f]);
-      qb[f] = fmaf(gdotf<EX, EY, EZ>(g1 + 3 * f), k.dt, si[f]);
-    }
-  } else {
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-      const float e = gdotf<EX, EY, EZ>(g1 + 3 * f) + gdotf<EX, EY, EZ>(g2 + 3 * f);
-      qa[f] = fmaf(-e, k.hdt, sc[f]);
-      qb[f] = fmaf(e, k.hdt, sc[f]);
-    }
-  }
-  const float fa = feq_dev(k, wgt, qa, edotf<EX, EY, EZ>(qa + 1));
-  const float fb = feq_dev(k, wgt, qb, -edotf<EX, EY, EZ>(qb + 1));
-  const float sum = fa + fb, dif = fa - fb;
-  if (EX) m[0] += EX > 0 ? dif : -dif;
-  if (EY) m[1] += EY > 0 ? dif : -dif;
-  if (EZ) m[2] += EZ > 0 ? dif : -dif;
-  if (diag) {
-    D += sum;
-  } else {
-    drhoI += sum;
-    if (EX) P[0] += sum;
-    if (EY) P[1] += sum;
-    if (EZ) P[2] += sum;
-  }
-  if (EX && EY) P[3] += (EX * EY > 0) ? sum : -sum;
-  if (EX && EZ) P[4] += (EX * EZ > 0) ? sum : -sum;
-  if (EY && EZ) P[5] += (EY * EZ > 0) ? sum : -sum;
-}
-
-// Face flux in deviation form (see the file comment); the same branches and
-// boundary handling as k_flux in kernels.cu.
+// Face flux in deviation form (see the file comment).
 // CR: the face's records from the compact tables (rec = its index there).
 template <bool CR>
 __device__ __forceinline__ void flux_face32(const KernelArgs& a, const int f, const int2 ids,
@@ -242,105 +103,20 @@ __device__ __forceinline__ void flux_face32(const KernelArgs& a, const int f, co
   const f4 f1 = CR ? ldf(a.frec1, rec) : ldf(a.face1, f);
   const f4 f2 = CR ? ldf(a.frec2, rec) : ldf(a.face2, f);
   const int o = ids.x, nb = ids.y;
-  const float n[3] = {f0.x, f0.y, f0.z};
-  const float area = f0.w, dt = f1.x;
+  const float n[3] = {f0.x, f0.y, f0.z}, dt = f1.x;
   const float t1[3] = {f1.y, f1.z, f1.w}, t2[3] = {f2.x, f2.y, f2.z};
   const f4 qo = ldf(a.state, o);
   float g1[12], g2[12], si[4], sn[4], sc[4];
   load_grad32(a.grad, o, g1);
-  const float qov[4] = {qo.w, qo.x, qo.y, qo.z};
-  bool interior = true;
-  f4 qn;
   if (nb < a.C) {
-    qn = ldf(a.state, nb);
+    const f4 qn = ldf(a.state, nb);
     load_grad32(a.grad, nb, g2);
+    interior_sides32(t1, t2, qo, qn, g1, g2, si, sn, sc);
   } else {
-    const int b = nb - a.C;
-    const f4 bv = ldf(a.bc0, b), tgt = ldf(a.bc1, b), dd = ldf(a.bc2, b), nm = ldf(a.bc3, b);
-    const int types = (int)nm.w;
-    ghost_grad32(qo, g1, bv, dd, nm, types, g2);
-    if (b == a.quirk_b) {
-      qn = ghost_state32(qo, tgt, types);  // interior branch, LBFS.cu:356
-    } else {
-      interior = false;
-      const int rt = types & 0xff, vt = types >> 8;
-      const float bvv[4] = {bv.w, bv.x, bv.y, bv.z};
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const bool dirichlet = (k == 0) ? (rt == 1) : (vt != 2);
-        sc[k] = dirichlet ? bvv[k]
-                          : qov[k] - (t1[0] * g2[3 * k] + t1[1] * g2[3 * k + 1] +
-                                      t1[2] * g2[3 * k + 2]);
-        si[k] = sc[k];
-        sn[k] = sc[k];
-      }
-#pragma unroll
-      for (int k = 0; k < 12; k++) g1[k] = g2[k];
-    }
+    boundary_sides32(a, nb - a.C, t1, t2, qo, g1, g2, si, sn, sc);
   }
-  if (interior) {
-    const float qnv[4] = {qn.w, qn.x, qn.y, qn.z};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      si[k] = qov[k] - (t1[0] * g1[3 * k] + t1[1] * g1[3 * k + 1] + t1[2] * g1[3 * k + 2]);
-      sn[k] = qnv[k] - (t2[0] * g2[3 * k] + t2[1] * g2[3 * k + 1] + t2[2] * g2[3 * k + 2]);
-      sc[k] = (si[k] + sn[k]) * 0.5f;
-    }
-  }
-  PairConst kc;
-  kc.d1 = 0.001f * dt;
-  kc.dt = dt;
-  kc.hdt = 0.5f * dt;
-  kc.rho0 = a.rho0f;
-  kc.U = (float)a.uref;
-  const float pg = (float)a.pg;
-  kc.c45u = 4.5f * kc.U * pg;
-  kc.c15u = 1.5f * kc.U * pg;
-  kc.u3 = 3.0f * kc.U;
-  kc.c45uu = kc.U * kc.c45u;
-  kc.c15uu = kc.U * kc.c15u;
-  const float w0 = 2.0f / 9.0f, w1 = 1.0f / 9.0f, w7 = 1.0f / 72.0f;
-  // centre node: e = 0
-  const float u2c = fmaf(sc[3], sc[3], fmaf(sc[2], sc[2], sc[1] * sc[1]));
-  float drhoI = w0 * fmaf(kc.rho0 + sc[0], kc.U * (-kc.c15u * u2c), sc[0]);
-  float m[3] = {0.0f, 0.0f, 0.0f};
-  float P[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-  float D = 0.0f;
-  lattice_pair32<1, 0, 0>(si, sn, sc, g1, g2, n, kc, w1, drhoI, m, P, D);
-  lattice_pair32<0, 1, 0>(si, sn, sc, g1, g2, n, kc, w1, drhoI, m, P, D);
-  lattice_pair32<0, 0, 1>(si, sn, sc, g1, g2, n, kc, w1, drhoI, m, P, D);
-#pragma unroll
-  for (int k = 0; k < 4; k++) {  // (gx, gy, gz) -> (gx + gy, gx - gy, gz), see gdotf
-    const float s1 = g1[3 * k] + g1[3 * k + 1], r1 = g1[3 * k] - g1[3 * k + 1];
-    const float s2 = g2[3 * k] + g2[3 * k + 1], r2 = g2[3 * k] - g2[3 * k + 1];
-    g1[3 * k] = s1;
-    g1[3 * k + 1] = r1;
-    g2[3 * k] = s2;
-    g2[3 * k + 1] = r2;
-  }
-  lattice_pair32<1, 1, 1>(si, sn, sc, g1, g2, n, kc, w7, drhoI, m, P, D);
-  lattice_pair32<1, 1, -1>(si, sn, sc, g1, g2, n, kc, w7, drhoI, m, P, D);
-  lattice_pair32<1, -1, 1>(si, sn, sc, g1, g2, n, kc, w7, drhoI, m, P, D);
-  lattice_pair32<-1, 1, 1>(si, sn, sc, g1, g2, n, kc, w7, drhoI, m, P, D);
-  drhoI += D;
-  P[0] += D;
-  P[1] += D;
-  P[2] += D;
-
-  const float tau = f2.w;  // 3 nu / (dt_s gamma), per face from the layout
-  const float mn = m[0] * n[0] + m[1] * n[1] + m[2] * n[2];
-  const float Pn[3] = {P[0] * n[0] + P[3] * n[1] + P[4] * n[2],
-                       P[3] * n[0] + P[1] * n[1] + P[5] * n[2],
-                       P[4] * n[0] + P[5] * n[1] + P[2] * n[2]};
-  const float mnr = mn / (kc.rho0 + drhoI) * pg;
-  const float p3 = drhoI * (1.0f / 3.0f);
-  const float sA = area * a.inv_uref_f;  // momentum flux is stored divided by U
-  f4 out;
-  out.x = ((1.0f - tau) * fmaf(m[0], mnr, p3 * n[0]) + tau * Pn[0]) * sA;
-  out.y = ((1.0f - tau) * fmaf(m[1], mnr, p3 * n[1]) + tau * Pn[1]) * sA;
-  out.z = ((1.0f - tau) * fmaf(m[2], mnr, p3 * n[2]) + tau * Pn[2]) * sA;
-  out.w = mn * area;
-  stf(a.flux, f, out);
+  const unsigned sides = face_sides32(n[0], n[1], n[2], __fmul_rn(0.001f, dt));
+  stf(a.flux, f, face_flux32(a, n, f0.w, f2.w, sides, dt, si, sn, sc, g1, g2));
 }
 
 // Persistent over the faces, next face's ids prefetched (as k_flux); six blocks
@@ -370,26 +146,6 @@ __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
-}
-
-// One cell's RK stage in deviation units (as rk_stage in flux_core.cuh).
-template <int RK>
-__device__ __forceinline__ void rk_stage32(const float dt, const float rho0, const f4& t0,
-                                           const f4& t1, const float R[4], f4& q, f4& acc) {
-  constexpr float alpha = (RK == 0 || RK == 3) ? 1.0f : 0.5f;
-  constexpr float beta = (RK == 0 || RK == 3) ? (1.0f / 6.0f) : (1.0f / 3.0f);
-  const float bdt = __fmul_rn(dt, beta);
-  const f4& b = RK == 0 ? t0 : t1;
-  acc = f4{fmaf(R[0], bdt, b.x), fmaf(R[1], bdt, b.y), fmaf(R[2], bdt, b.z),
-           fmaf(R[3], bdt, b.w)};
-  f4 f = acc;
-  if (RK != 3) {
-    const float adt = __fmul_rn(dt, alpha);
-    f = f4{fmaf(R[0], adt, t0.x), fmaf(R[1], adt, t0.y), fmaf(R[2], adt, t0.z),
-           fmaf(R[3], adt, t0.w)};
-  }
-  const float rho = __fadd_rn(rho0, f.w);
-  q = f4{__fdiv_rn(f.x, rho), __fdiv_rn(f.y, rho), __fdiv_rn(f.z, rho), f.w};
 }
 
 // Gather + body force + RK stage in deviation units; the last stage reduces

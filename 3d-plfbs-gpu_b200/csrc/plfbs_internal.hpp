@@ -335,6 +335,7 @@ struct KernelArgs {
   const int32_t* face_ids;                     // int2 [F]
   float* fforce_x; float* fforce_y; float* fforce_z;  // [C] body force / U, or null
   float rho0f, inv_uref_f;
+  float eq32_k0, eq32_k1, eq32_cd, eq32_pgcd;  // flux_core32.cuh; pgcd = cd / gamma
   // host side: tensor maps of the TMA-staged FP64 flux kernel, or null for
   // the per-thread gathers (read by launch_flux, not by kernels)
   const FluxMaps* flux_maps;
