@@ -178,6 +178,9 @@ void give_pinned_staging(void* p, size_t n) {
 
 
 // One time step: IBM, then 4 x (gradient, flux, update) (Solver_gpu.cu:667-833).
+// Whether a run takes the march kernel instead of the step graph.
+bool marches(const KernelArgs& a) { return a.tiles.n > 0 && !a.flux_maps && !a.res_debug; }
+
 void enqueue_step(const KernelArgs& a, int prec, cudaStream_t s) {
   plfbs::launch_ibm(a, prec, s);
   for (int rk = 0; rk < 4; rk++) {
@@ -192,6 +195,7 @@ int capture_step(plfbs_ctx* ctx) {
     cudaGraphExecDestroy(ctx->step_exec);
     ctx->step_exec = nullptr;
   }
+  if (marches(ctx->args)) return PLFBS_OK;  // no graph
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   enqueue_step(ctx->args, ctx->cfg.precision, ctx->stream);
@@ -610,6 +614,10 @@ int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh, const plf
     NvtxRange r("compact layout");
     if ((rc = build_compact_layout(ctx))) return fail(rc);
   }
+  {
+    NvtxRange r("tiles");
+    if ((rc = build_tiles(ctx))) return fail(rc);
+  }
   if (ctx->pre.bc[0]) {  // copied while the mesh copies ran
     a.bc0 = ctx->pre.bc[0];
     a.bc1 = ctx->pre.bc[1];
@@ -636,7 +644,10 @@ int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh, const plf
     if ((rc = dev_upload(ctx, &p, L.bc3))) return fail(rc);
     a.bc3 = p;
   }
-  if ((rc = dev_alloc(ctx, &p, (size_t)a.nblk_update * 4 * sizeof(double)))) return fail(rc);
+  {  // residual partial sums: per block, or per warp for a context that marches
+    const size_t n = a.red_order ? ((size_t)L.C + 31) / 32 : (size_t)a.nblk_update;
+    if ((rc = dev_alloc(ctx, &p, n * 4 * sizeof(double)))) return fail(rc);
+  }
   a.partial = static_cast<double*>(p);
   if ((rc = dev_alloc(ctx, &p, sizeof(DevStats)))) return fail(rc);
   a.stats = static_cast<DevStats*>(p);
@@ -741,6 +752,7 @@ int plfbs_wall_forces(plfbs_ctx* ctx, const int32_t* wall_bc, int32_t n_wall, do
       return set_err(ctx, PLFBS_ERR_BC, "wall faces need velocity type 1 (Dirichlet) or 2 (Neumann)");
     walls[4 + k] = b;
   }
+  ctx->grad_stale = false;  // the gradients below are the current state's
   // wall_buf: ints [0, 4) zero (a halt flag that reads 0), [4, 4 + n) the
   // walls, then (16-byte aligned) the two sums
   const size_t sums_at = ((size_t)(n_wall + 4) * sizeof(int) + 15) & ~(size_t)15;
@@ -1044,7 +1056,10 @@ int plfbs_run(plfbs_ctx* ctx, int64_t max_steps, plfbs_stats* stats, double* his
     const long long n = std::min<long long>(batch, max_steps - done);
     NvtxRange r("step batch");
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    for (long long k = 0; k < n; k++) CK(cudaGraphLaunch(ctx->step_exec, ctx->stream));
+    if (marches(ctx->args))
+      CK(plfbs::launch_march(ctx->args, ctx->cfg.precision, (int)n, ctx->stream));
+    else
+      for (long long k = 0; k < n; k++) CK(cudaGraphLaunch(ctx->step_exec, ctx->stream));
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
     TRY(wait_steps(ctx, ctx->timeout_s));
     TRY(read_stats(ctx));
@@ -1067,6 +1082,7 @@ int plfbs_run(plfbs_ctx* ctx, int64_t max_steps, plfbs_stats* stats, double* his
     halt = ctx->stats_host->halt != 0;
     if (now - start == done && !halt)  // a batch that advanced nothing: never wait again
       return set_err(ctx, PLFBS_ERR_STATE, "the step graph made no progress");
+    if (now > start + done && marches(ctx->args)) ctx->grad_stale = ctx->flux_stale = true;
     done = now - start;
   }
   CK(cudaGetLastError());
@@ -1208,6 +1224,7 @@ int plfbs_set_debug(plfbs_ctx* ctx, int enable) {
 int plfbs_run_stages(plfbs_ctx* ctx, int64_t n_stages) {
   TRY(check_ctx(ctx));
   if (!ctx->have_state) return set_err(ctx, PLFBS_ERR_STATE, "run_stages before set_state");
+  if (n_stages > 0) ctx->grad_stale = ctx->flux_stale = false;
   for (int64_t g = 0; g < n_stages; g++) {
     const int rk = (int)(ctx->stages_done % 4);
     if (rk == 0) plfbs::launch_ibm(ctx->args, ctx->cfg.precision, ctx->stream);
@@ -1222,10 +1239,35 @@ int plfbs_run_stages(plfbs_ctx* ctx, int64_t n_stages) {
   return check_fault(ctx);
 }
 
+// The gradients and fluxes of the last stage of a march, recomputed from its input
+// state (state2 holds it until the next step).
+static int refresh_introspection(plfbs_ctx* ctx) {
+  if (!ctx->grad_stale && !ctx->flux_stale) return PLFBS_OK;
+  const int prec = ctx->cfg.precision;
+  void* zero = nullptr;  // a halt flag that reads 0: a halted context's kernels return at entry
+  TRY(scratch_alloc(ctx, &zero, sizeof(DevStats)));
+  cudaError_t e = cudaMemsetAsync(zero, 0, sizeof(DevStats), ctx->stream);
+  KernelArgs a = ctx->args;
+  a.stats = static_cast<DevStats*>(zero);
+  KernelArgs b = a;
+  b.state = a.state2;
+  b.flux_maps = nullptr;
+  plfbs::launch_gradient(b, prec, ctx->stream);
+  if (ctx->flux_stale) plfbs::launch_flux(b, prec, ctx->stream);
+  // a wall-force call since has left the current state's gradients
+  if (!ctx->grad_stale) plfbs::launch_gradient(a, prec, ctx->stream);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  scratch_free(ctx, zero);
+  CK(e);
+  ctx->grad_stale = ctx->flux_stale = false;
+  return PLFBS_OK;
+}
+
 int plfbs_get_gradients(plfbs_ctx* ctx, double* grad, int32_t n_cells) {
   TRY(check_ctx(ctx));
   const Layout& L = ctx->L;
   if (!grad || n_cells != L.C) return set_err(ctx, PLFBS_ERR_ARG, "gradients: need 12 n_cells");
+  TRY(refresh_introspection(ctx));
   std::vector<double> g(12 * (size_t)L.C);
   if (ctx->cfg.precision == PLFBS_FP32_DEVIATION) {
     std::vector<float> f(g.size());
@@ -1248,6 +1290,7 @@ int plfbs_get_face_flux(plfbs_ctx* ctx, double* flux, int32_t n_faces) {
   TRY(check_ctx(ctx));
   const Layout& L = ctx->L;
   if (!flux || n_faces != L.F) return set_err(ctx, PLFBS_ERR_ARG, "face flux: need 4 n_faces");
+  TRY(refresh_introspection(ctx));
   std::vector<double> g;
   TRY(download4(ctx, ctx->args.flux, (size_t)L.F, g, true));
   std::vector<int32_t> order(L.F);
@@ -1326,6 +1369,7 @@ int plfbs_profile_steps(plfbs_ctx* ctx, int64_t n_steps, double* ms) {
   if (!ms) return set_err(ctx, PLFBS_ERR_ARG, "null output");
   if (!ctx->have_state || ctx->stages_done != 0)
     return set_err(ctx, PLFBS_ERR_STATE, "profile needs a state at a step boundary");
+  if (n_steps > 0) ctx->grad_stale = ctx->flux_stale = false;
   for (int k = 0; k < 4; k++) ms[k] = 0.0;
   // ev[0] before the IBM kernel, ev[1] after it, ev[2 + 3 rk + j] after kernel j
   // (gradient, flux, update) of stage rk: 14 events in all
@@ -1374,6 +1418,7 @@ int plfbs_profile_kernels(plfbs_ctx* ctx, int64_t launches, double* ms) {
   TRY(read_stats(ctx));
   if (ctx->stats_host->halt)
     return set_err(ctx, PLFBS_ERR_STATE, "the run has halted: its kernels return at entry");
+  ctx->grad_stale = ctx->flux_stale = false;
   for (int k = 0; k < 5; k++) ms[k] = 0.0;
   // everything the launches write that a later step reads, copied aside on
   // the device and put back afterwards (flux, gradients and partial sums are

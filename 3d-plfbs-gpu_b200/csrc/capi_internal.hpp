@@ -38,6 +38,10 @@ struct plfbs_ctx {
   int compact_faces = 0;          // unique face records in the compact layout (0: none)
   int compact_cells = 0;          // unique cell weight sets in the compact layout (0: none)
   bool flux_maps_ok = false;
+  int32_t* curve = nullptr;       // device [C]: the cells along a space-filling curve
+  // gradients and fluxes on the device are older than the last step (the
+  // march kernel does not write them); recomputed when asked for
+  bool grad_stale = false, flux_stale = false;
   // The caller's mesh arrays, copied to the device at the start of
   // plfbs_create, checked there (launch_mesh_scan) and read by the layout
   // only after the checks passed: owner, neighbour [F] int; area, sdt [F],
@@ -121,6 +125,9 @@ int prestage_layout(plfbs_ctx* ctx);
 void release_staging(plfbs_ctx* ctx);
 void free_stage(plfbs_ctx* ctx);
 int build_compact_layout(plfbs_ctx* ctx);
+// The tile tables of the march kernel (KernelArgs::tiles; none for a mesh that
+// does not fit one tile per SM).
+int build_tiles(plfbs_ctx* ctx);
 
 // The renumber-1 cell order (reverse Cuthill-McKee, order[new] = caller cell)
 // built on the device (renumber 2; capi_layout.cpp).

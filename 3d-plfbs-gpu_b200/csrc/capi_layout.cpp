@@ -189,6 +189,26 @@ int build_device_layout(plfbs_ctx* ctx, const plfbs_mesh_view& m) {
   ctx->perm = static_cast<int32_t*>(p);
   plfbs::launch_perm(d.cell_new, d.bc_new, L.C, L.B, ctx->perm, ctx->stream);
   CK(cudaGetLastError());
+  // the cells along a space-filling curve, for the tiles of a mesh small
+  // enough to have them (build_tiles)
+  if (L.C <= plfbs::march_max_tiles() * plfbs::march_max_own()) {
+    const plfbs::CurveSizes z = plfbs::curve_sizes(L.C);
+    plfbs::CurveScratch c{};
+    TRY(S.alloc(&c.part, 8 * z.part, false));
+    for (int k = 0; k < 2; k++) {
+      TRY(S.alloc(&c.key[k], 4 * C, false));
+      TRY(S.alloc(&c.val[k], 4 * C, false));
+    }
+    TRY(S.alloc(&c.count, 4 * z.count, false));
+    TRY(S.alloc(&c.off, 4 * z.count, false));
+    TRY(S.alloc(&c.wsum, 4 * z.windows, false));
+    TRY(S.alloc(&c.wbase, 4 * (z.windows + 1), false));
+    TRY(S.alloc(&c.info, 16, true));
+    TRY(pool_alloc(ctx, &p, 4 * C));
+    ctx->curve = static_cast<int32_t*>(p);
+    plfbs::launch_cell_curve(d, c, ctx->curve, ctx->stream);
+    CK(cudaGetLastError());
+  }
   plfbs::LayoutScratch s{};
   TRY(S.alloc(&s.own_cnt, 4 * C, true));
   TRY(S.alloc(&s.own_off, 4 * C, false));
@@ -348,6 +368,86 @@ int device_cell_order(plfbs_ctx* ctx, const plfbs_mesh_view& m, std::vector<int3
   return PLFBS_OK;
 }
 
+// One tile per SM, so the mesh must fit them all at once: a tile's rows in a
+// block's shared memory and its indices in the tables' widths (up to about
+// 68,000 FP64 or 142,000 FP32 hexahedra on 148 SMs). Within that the march wins
+// where the face records are few and shared (FP64 hexahedra: 512 cells 25 us
+// per step against 57 with the kernels one by one, 27,648 cells 41 : 76, 64,000
+// cells 64 : 86; FP32 128,000 cells 70 : 85). With records of their own its
+// blocks wait for them at every face, so it takes the mesh up to
+// kMarchFaces64 / kMarchFaces32 faces per SM (FP64: 131,000 faces 70 us : 78, but
+// 170,000 90 : 82; FP32: 170,000 55 : 64, 320,000 153 : 78).
+constexpr int kMarchFaces64 = 900, kMarchFaces32 = 1600;
+int build_tiles(plfbs_ctx* ctx) {
+  KernelArgs& a = ctx->args;
+  const int prec = ctx->cfg.precision;
+  int sms = 0, coop = 0, most_smem = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+  CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
+  CK(cudaDeviceGetAttribute(&most_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+  most_smem -= 4096;  // the kernel's own arrays
+  const int tiles = std::min(sms, plfbs::march_max_tiles());
+  plfbs::TileArgs t{};
+  t.T = ((a.C + tiles - 1) / tiles + 31) / 32 * 32;
+  if (!coop || t.T > plfbs::march_max_own() || a.F >= (1 << 28) || !ctx->curve)
+    return PLFBS_OK;
+  const bool shared = a.face_rec && a.wtab;  // the compact layout
+  if (!shared &&
+      a.F > tiles * (prec == PLFBS_FP32_DEVIATION ? kMarchFaces32 : kMarchFaces64))
+    return PLFBS_OK;
+  t.n = (a.C + t.T - 1) / t.T;
+  ScratchList S(ctx);
+  int32_t *most = nullptr, *pos = nullptr;
+  uint16_t* side = nullptr;
+  TRY(S.alloc(&most, 8, true));
+  TRY(S.alloc(&side, 2 * (size_t)a.F, false));
+  TRY(S.alloc(&pos, 4 * (size_t)a.C, false));
+  plfbs::launch_tile_order(a.C, t.T, ctx->curve, pos, ctx->stream);
+  plfbs::launch_tile_count(a, ctx->curve, pos, t.T, most, ctx->stream);
+  plfbs::launch_face_sides(a, prec, side, ctx->stream);
+  CK(cudaGetLastError());
+  int32_t got[2];
+  CK(cudaMemcpyAsync(got, most, 8, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  t.SC = (t.T + got[1] + 31) / 32 * 32;
+  t.SF = (got[0] + 31) / 32 * 32;
+  t.smem = plfbs::march_smem(a, prec, most_smem, t);
+  if (t.T + got[1] > plfbs::kTileMaxCells || got[0] > plfbs::kTileMaxFaces || t.smem == 0)
+    return PLFBS_OK;
+  const size_t cells = (size_t)t.n * t.SC, faces = (size_t)t.n * t.SF;
+  void* p = nullptr;
+  TRY(pool_alloc(ctx, &p, 4 * cells));
+  t.cell = static_cast<int32_t*>(p);
+  TRY(pool_alloc(ctx, &p, 4 * cells * std::max(a.K, 1)));
+  t.nbr = static_cast<int32_t*>(p);
+  if (a.cell_wset) {
+    TRY(pool_alloc(ctx, &p, 4 * cells));
+    t.wset = static_cast<int32_t*>(p);
+  }
+  TRY(pool_alloc(ctx, &p, 4 * faces));
+  t.ij = static_cast<uint32_t*>(p);
+  TRY(pool_alloc(ctx, &p, 4 * faces));
+  t.fid = static_cast<int32_t*>(p);
+  if (a.face_rec) {
+    TRY(pool_alloc(ctx, &p, 4 * faces));
+    t.rec = static_cast<int32_t*>(p);
+  }
+  TRY(pool_alloc(ctx, &p, 2 * (size_t)t.n * t.T * std::max(a.K2, 1)));
+  t.slot = static_cast<uint16_t*>(p);
+  TRY(pool_alloc(ctx, &p, sizeof(int2) * (size_t)t.n));
+  t.count = static_cast<int2*>(p);
+  TRY(pool_alloc(ctx, &p, (prec == PLFBS_FP32_DEVIATION ? 16 : 32) * ((size_t)a.C + a.B)));
+  a.state2 = p;
+  TRY(pool_alloc(ctx, &p, sizeof(unsigned)));
+  a.grid_bar = static_cast<unsigned*>(p);
+  plfbs::launch_tile_build(a, ctx->curve, pos, side, t, got[0], got[1], ctx->stream);
+  CK(cudaGetLastError());
+  a.tiles = t;
+  a.red_order = ctx->curve;
+  a.red_warps = t.T / 32;
+  return PLFBS_OK;
+}
+
 // The compact layout: face records and cells' weight sets that are
 // bitwise equal are stored once (layout.cu, dedupe), each item keeping an
 // index. Used where a table holds at most 1/8 of the items (structured
@@ -404,9 +504,12 @@ int build_compact_layout(plfbs_ctx* ctx) {
       a.frec0 = t[0];
       a.frec1 = t[1];
       a.frec2 = t[2];
-      ctx->compact_faces = U;
-      if (!fp32) {
-        TRY(pool_alloc(ctx, &p, 4 * (size_t)U));
+      ctx->compact_faces = a.n_frec = U;
+      TRY(pool_alloc(ctx, &p, 4 * (size_t)U));
+      if (fp32) {
+        plfbs::launch_record_sides32(t[0], t[1], U, static_cast<int32_t*>(p), ctx->stream);
+        a.frec_sides = static_cast<const int32_t*>(p);
+      } else {
         void* relax = nullptr;
         TRY(pool_alloc(ctx, &relax, 16 * (size_t)U));
         plfbs::launch_record_sides(t[0], t[1], t[2], a.eq_cd, U, ctx->cfg.flavour,
@@ -420,7 +523,7 @@ int build_compact_layout(plfbs_ctx* ctx) {
       plfbs::launch_dedupe_emit(src[k], d[k], index, p, nullptr, nullptr, ctx->stream);
       a.cell_wset = index;
       a.wtab = p;
-      ctx->compact_cells = U;
+      ctx->compact_cells = a.n_wset = U;
     }
   }
   CK(cudaGetLastError());

@@ -23,7 +23,7 @@
 #include <cstdint>
 
 #include "flux_core.cuh"
-#include "ibm_spread.cuh"
+#include "ibm_core.cuh"
 #include "plfbs_internal.hpp"
 
 namespace plfbs {
@@ -328,8 +328,10 @@ __device__ __forceinline__ double warp_sum(double v) {
 // K2MAX: face slots the launch is specialised for (0 = any count, looped).
 template <int RK, int K2MAX>
 __global__ void __launch_bounds__(kBlock) k_update(const KernelArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (halted(a)) return;  // uniform across the launch
+  // a context that marches sums its residuals along its tiles
+  if (RK == 3 && a.red_order) i = i < a.C ? __ldg(a.red_order + i) : a.C;
   double sq[4] = {0.0, 0.0, 0.0, 0.0};
   bool bad = false;
   if (i < a.C) {
@@ -371,14 +373,14 @@ __global__ void __launch_bounds__(kBlock) k_update(const KernelArgs a) {
       }
     }
     const double iv = __ldg(static_cast<const double*>(a.inv_volume) + i);
-    double R[4] = {r[0] * iv, r[1] * iv, r[2] * iv, r[3] * iv};  // u, v, w, rho
+    double fc[3] = {a.pressure_gradient, 0.0, 0.0};
     if (a.force_x) {
-      R[0] += a.force_x[i];
-      R[1] += a.force_y[i];
-      R[2] += a.force_z[i];
-    } else {
-      R[0] += a.pressure_gradient;
+      fc[0] = a.force_x[i];
+      fc[1] = a.force_y[i];
+      fc[2] = a.force_z[i];
     }
+    const double R[4] = {fma(r[0], iv, fc[0]), fma(r[1], iv, fc[1]), fma(r[2], iv, fc[2]),
+                         r[3] * iv};  // u, v, w, rho
     if (a.res_debug) st4(a.res_debug, i, d4{R[0], R[1], R[2], R[3]});
     d4 q, acc;
     rk_stage<RK>(a.dt, t0, t1, R, q, acc);
@@ -416,7 +418,11 @@ __global__ void __launch_bounds__(kBlock) k_update(const KernelArgs a) {
     if (lane == 0) red[warp][c] = v;
   }
   __syncthreads();
-  if (threadIdx.x < 4) {
+  if (a.red_order) {  // per warp of cells; k_finish adds them tile by tile
+    const int w = threadIdx.x / 4, c = threadIdx.x & 3;
+    const long long at = (long long)blockIdx.x * (kBlock / 32) + w;
+    if (w < kBlock / 32 && 32 * at < a.C) a.partial[4 * at + c] = red[w][c];
+  } else if (threadIdx.x < 4) {
     double v = 0.0;
     for (int w = 0; w < kBlock / 32; w++) v += red[w][threadIdx.x];
     a.partial[4LL * blockIdx.x + threadIdx.x] = v;
@@ -433,8 +439,18 @@ __global__ void __launch_bounds__(kFinishBlock) k_finish(const KernelArgs a) {
   __shared__ double red[kFinishBlock / 32][4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double v[4] = {0.0, 0.0, 0.0, 0.0};
+  if (a.red_order) {  // tile by tile, its warps in order
+    const int nw = (a.C + 31) / 32;
+    for (int b = threadIdx.x; b < a.tiles.n; b += kFinishBlock)
+      for (int c = 0; c < 4; c++) {
+        double s = 0.0;
+        for (int w = b * a.red_warps; w < min((b + 1) * a.red_warps, nw); w++)
+          s += a.partial[4 * w + c];
+        v[c] += s;
+      }
+  }
 #pragma unroll 4
-  for (int b = threadIdx.x; b < a.nblk_update; b += kFinishBlock) {
+  for (int b = threadIdx.x; b < (a.red_order ? 0 : a.nblk_update); b += kFinishBlock) {
     const double2 p0 = __ldg(reinterpret_cast<const double2*>(a.partial + 4LL * b));
     const double2 p1 = __ldg(reinterpret_cast<const double2*>(a.partial + 4LL * b) + 1);
     v[0] += p0.x;
@@ -493,90 +509,10 @@ __global__ void k_seed(const KernelArgs a) {
   st4(a.t0, i, q);
 }
 
-// ---------------------------------------------------------------------------
-// IBM (immersed_boundary_method.cu:13-90, 161-190, 244-295, 299-375), once
-// per time step before the RK stages.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void stencil_origin(const KernelArgs& a, const double x[3],
-                                               double r[3], int lo[3]) {
-  r[0] = (x[0] - a.origin[0]) / a.ibm_dx;
-  r[1] = fabs((x[1] - a.origin[1]) / a.ibm_dx);
-  r[2] = fabs((x[2] - a.origin[2]) / a.ibm_dx);
-#pragma unroll
-  for (int c = 0; c < 3; c++) lo[c] = (int)round(r[c]) - 1;
-}
-
-// Eight threads per node, one per cell of its 2 x 2 x 2 stencil: each loads
-// its cell's state, the node's velocity is the sum over the eight (xor
-// butterfly, so every lane holds the same bits), every lane advances the node
-// and forms its force, and the warp spreads its lanes' forces with one FP64
-// atomic per distinct cell and component (spread_aggregated; nodes in the
-// spatial order ibm_order). Lane 0 of a node writes the node's arrays.
+// The immersed body (ibm_core.cuh), once per time step before the RK stages.
 __global__ void __launch_bounds__(kIbmBlock) k_ibm(const KernelArgs a) {
   if (halted(a)) return;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int slot = t >> 3, sub = t & 7;
-  const bool active = slot < a.N;
-  const int nd = active ? __ldg(a.ibm_order + slot) : 0;
-  const int xc = a.ibm_xc, yc = a.ibm_yc;
-  double x[3] = {0.0, 0.0, 0.0}, r[3] = {0.0, 0.0, 0.0};
-  int lo[3] = {0, 0, 0};
-  if (active) {
-#pragma unroll
-    for (int c = 0; c < 3; c++) x[c] = a.node_x[3 * nd + c];
-    stencil_origin(a, x, r, lo);
-  }
-  const int di = sub & 1, dj = (sub >> 1) & 1, dk = sub >> 2;
-  double v[3] = {0.0, 0.0, 0.0};
-  {
-    const int ii = lo[0] + di, jj = lo[1] + dj, kk = lo[2] + dk;
-    const long long cell = (long long)ii + (long long)jj * xc + (long long)kk * yc * xc;
-    if (active && cell < a.C && cell >= 0) {  // the reference's linear-index check
-      const double wx = 1 - fabs(ii + 0.5 - r[0]);
-      const double wy = 1 - fabs(jj + 0.5 - r[1]);
-      const double wz = 1 - fabs(kk + 0.5 - r[2]);
-      const d4 q = ld4(a.state, a.ibm_map[cell]);
-      v[0] = q.x * wx * wy * wz * a.ibm_inv_dx3;
-      v[1] = q.y * wx * wy * wz * a.ibm_inv_dx3;
-      v[2] = q.z * wx * wy * wz * a.ibm_inv_dx3;
-    }
-  }
-  const unsigned full = 0xffffffffu;
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1)
-#pragma unroll
-    for (int c = 0; c < 3; c++) v[c] += __shfl_xor_sync(full, v[c], o);
-  const unsigned act = __ballot_sync(full, active);
-  if (!active) return;
-  double fn[3];
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    x[c] = a.node_x0[3 * nd + c] + v[c] * a.dt;
-    fn[c] = -a.ibm_area_k * (x[c] - a.node_ref[3 * nd + c]);
-  }
-  if (sub == 0) {
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      a.node_x[3 * nd + c] = x[c];
-      a.node_x0[3 * nd + c] = x[c];
-      a.node_vel[3 * nd + c] = v[c];
-      a.node_force[3 * nd + c] = fn[c];
-    }
-  }
-  stencil_origin(a, x, r, lo);
-  const int ii = lo[0] + di, jj = lo[1] + dj, kk = lo[2] + dk;
-  const long long cell = (long long)ii + (long long)jj * xc + (long long)kk * yc * xc;
-  int target = -1;
-  double f[3] = {0.0, 0.0, 0.0};
-  if (cell < a.C && cell >= 0) {
-    const double wx = 1 - fabs(ii + 0.5 - r[0]);
-    const double wy = 1 - fabs(jj + 0.5 - r[1]);
-    const double wz = 1 - fabs(kk + 0.5 - r[2]);
-    target = a.ibm_map[cell];
-#pragma unroll
-    for (int c = 0; c < 3; c++) f[c] = fn[c] * wx * wy * wz * a.ibm_inv_dx3;
-  }
-  spread_aggregated(act, target, f, a.force_x, a.force_y, a.force_z);
+  ibm_thread(a, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -770,7 +706,8 @@ void launch_flux(const KernelArgs& a, int precision, cudaStream_t s) {
   }
 }
 template <int RK>
-static void launch_update_rk(const KernelArgs& a, int nb, cudaStream_t s) {
+static void launch_update_rk(const KernelArgs& a, cudaStream_t s) {
+  const int nb = blocks_for(a.C, kBlock);
   if (a.K2 <= 4)
     k_update<RK, 4><<<nb, kBlock, 0, s>>>(a);
   else if (a.K2 <= 6)
@@ -782,13 +719,12 @@ static void launch_update_rk(const KernelArgs& a, int nb, cudaStream_t s) {
 }
 void launch_update(const KernelArgs& a, int precision, int rk, cudaStream_t s, bool finish) {
   if (precision == PLFBS_FP32_DEVIATION) return launch_update32(a, rk, s, finish);
-  const int nb = blocks_for(a.C, kBlock);
   switch (rk) {
-    case 0: launch_update_rk<0>(a, nb, s); break;
-    case 1: launch_update_rk<1>(a, nb, s); break;
-    case 2: launch_update_rk<2>(a, nb, s); break;
+    case 0: launch_update_rk<0>(a, s); break;
+    case 1: launch_update_rk<1>(a, s); break;
+    case 2: launch_update_rk<2>(a, s); break;
     default:
-      launch_update_rk<3>(a, nb, s);
+      launch_update_rk<3>(a, s);
       if (finish) k_finish<<<1, kFinishBlock, 0, s>>>(a);
       break;
   }

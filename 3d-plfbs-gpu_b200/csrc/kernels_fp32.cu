@@ -20,7 +20,7 @@
 #include <cstdint>
 
 #include "flux_core32.cuh"
-#include "ibm_spread.cuh"
+#include "ibm_core.cuh"
 #include "plfbs_internal.hpp"
 
 namespace plfbs {
@@ -153,8 +153,9 @@ __device__ __forceinline__ double warp_sum(double v) {
 // so inv_ref_mom is 1 / rho_ref here).
 template <int RK, int K2MAX>
 __global__ void __launch_bounds__(kBlock) k_update32(const KernelArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (halted(a)) return;
+  if (RK == 3 && a.red_order) i = i < a.C ? __ldg(a.red_order + i) : a.C;  // as k_update
   double sq[4] = {0.0, 0.0, 0.0, 0.0};
   bool bad = false;
   if (i < a.C) {
@@ -182,15 +183,15 @@ __global__ void __launch_bounds__(kBlock) k_update32(const KernelArgs a) {
       r[3] = fmaf(sg, fl[k].w, r[3]);
     }
     const float iv = __ldg(static_cast<const float*>(a.inv_volume) + i);
-    float R[4] = {r[0] * iv, r[1] * iv, r[2] * iv, r[3] * iv};
-    const float pgU = (float)(a.pressure_gradient) * a.inv_uref_f;
+    const float pgU = __fmul_rn((float)a.pressure_gradient, a.inv_uref_f);
+    float fc[3] = {pgU, 0.0f, 0.0f};
     if (a.fforce_x) {
-      R[0] += a.fforce_x[i];
-      R[1] += a.fforce_y[i];
-      R[2] += a.fforce_z[i];
-    } else {
-      R[0] += pgU;
+      fc[0] = a.fforce_x[i];
+      fc[1] = a.fforce_y[i];
+      fc[2] = a.fforce_z[i];
     }
+    const float R[4] = {fmaf(r[0], iv, fc[0]), fmaf(r[1], iv, fc[1]), fmaf(r[2], iv, fc[2]),
+                        r[3] * iv};
     if (a.res_debug) stf(a.res_debug, i, f4{R[0], R[1], R[2], R[3]});
     f4 q, acc;
     rk_stage32<RK>((float)a.dt, a.rho0f, t0, t1, R, q, acc);
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(kBlock) k_update32(const KernelArgs a) {
       sq[1] = (double)R[0] * R[0];
       sq[2] = (double)R[1] * R[1];
       sq[3] = (double)R[2] * R[2];
-      bad = !(a.rho0f + acc.w <= 1000.0f);
+      bad = !(__fadd_rn(a.rho0f, acc.w) <= 1000.0f);
     }
     stf(RK == 3 ? a.t0 : a.t1, i, acc);
     stf(a.state, i, q);
@@ -225,7 +226,11 @@ __global__ void __launch_bounds__(kBlock) k_update32(const KernelArgs a) {
     if (lane == 0) red[warp][c] = v;
   }
   __syncthreads();
-  if (threadIdx.x < 4) {
+  if (a.red_order) {  // per warp of cells; k_finish adds them tile by tile
+    const int w = threadIdx.x / 4, c = threadIdx.x & 3;
+    const long long at = (long long)blockIdx.x * (kBlock / 32) + w;
+    if (w < kBlock / 32 && 32 * at < a.C) a.partial[4 * at + c] = red[w][c];
+  } else if (threadIdx.x < 4) {
     double v = 0.0;
     for (int w = 0; w < kBlock / 32; w++) v += red[w][threadIdx.x];
     a.partial[4LL * blockIdx.x + threadIdx.x] = v;
@@ -242,8 +247,18 @@ __global__ void __launch_bounds__(kFinishBlock) k_finish32(const KernelArgs a) {
   __shared__ double red[kFinishBlock / 32][4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double v[4] = {0.0, 0.0, 0.0, 0.0};
+  if (a.red_order) {  // tile by tile, its warps in order
+    const int nw = (a.C + 31) / 32;
+    for (int b = threadIdx.x; b < a.tiles.n; b += kFinishBlock)
+      for (int c = 0; c < 4; c++) {
+        double s = 0.0;
+        for (int w = b * a.red_warps; w < min((b + 1) * a.red_warps, nw); w++)
+          s += a.partial[4 * w + c];
+        v[c] += s;
+      }
+  }
 #pragma unroll 4
-  for (int b = threadIdx.x; b < a.nblk_update; b += kFinishBlock) {
+  for (int b = threadIdx.x; b < (a.red_order ? 0 : a.nblk_update); b += kFinishBlock) {
     const double2 p0 = __ldg(reinterpret_cast<const double2*>(a.partial + 4LL * b));
     const double2 p1 = __ldg(reinterpret_cast<const double2*>(a.partial + 4LL * b) + 1);
     v[0] += p0.x;
@@ -303,88 +318,24 @@ __global__ void k_seed32(const KernelArgs a) {
   stf(a.t0, i, q);
 }
 
-// IBM with FP64 node positions and forces; velocities interpolated from the
-// FP32 state (times U) and forces spread as force / U in FP32.
-// Eight threads per node, warp-aggregated spreading (as k_ibm). Node quantities stay FP64; the state is
-// scaled by U when read and the spread force divided by U when written.
 __global__ void __launch_bounds__(kIbmBlock) k_ibm32(const KernelArgs a) {
   if (halted(a)) return;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int slot = t >> 3, sub = t & 7;
-  const bool active = slot < a.N;
-  const int nd = active ? __ldg(a.ibm_order + slot) : 0;
-  const int xc = a.ibm_xc, yc = a.ibm_yc;
-  const double U = a.uref;
-  double x[3] = {0.0, 0.0, 0.0}, r[3] = {0.0, 0.0, 0.0};
-  int lo[3] = {0, 0, 0};
-  auto origin = [&](const double p[3]) {
-    r[0] = (p[0] - a.origin[0]) / a.ibm_dx;
-    r[1] = fabs((p[1] - a.origin[1]) / a.ibm_dx);
-    r[2] = fabs((p[2] - a.origin[2]) / a.ibm_dx);
-#pragma unroll
-    for (int c = 0; c < 3; c++) lo[c] = (int)round(r[c]) - 1;
-  };
-  if (active) {
-#pragma unroll
-    for (int c = 0; c < 3; c++) x[c] = a.node_x[3 * nd + c];
-    origin(x);
+  ibm_thread32(a, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// Branch bits of the compact layout's unique records.
+__global__ void k_record_sides32(const void* frec0, const void* frec1, int n, int32_t* out) {
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+    const f4 f0 = ldf(frec0, r);
+    out[r] = (int32_t)face_sides32(f0.x, f0.y, f0.z, __fmul_rn(0.001f, ldf(frec1, r).x));
   }
-  const int di = sub & 1, dj = (sub >> 1) & 1, dk = sub >> 2;
-  double v[3] = {0.0, 0.0, 0.0};
-  {
-    const int ii = lo[0] + di, jj = lo[1] + dj, kk = lo[2] + dk;
-    const long long cell = (long long)ii + (long long)jj * xc + (long long)kk * yc * xc;
-    if (active && cell < a.C && cell >= 0) {
-      const double wx = 1 - fabs(ii + 0.5 - r[0]);
-      const double wy = 1 - fabs(jj + 0.5 - r[1]);
-      const double wz = 1 - fabs(kk + 0.5 - r[2]);
-      const f4 q = ldf(a.state, a.ibm_map[cell]);
-      v[0] = (U * q.x) * wx * wy * wz * a.ibm_inv_dx3;
-      v[1] = (U * q.y) * wx * wy * wz * a.ibm_inv_dx3;
-      v[2] = (U * q.z) * wx * wy * wz * a.ibm_inv_dx3;
-    }
-  }
-  const unsigned full = 0xffffffffu;
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1)
-#pragma unroll
-    for (int c = 0; c < 3; c++) v[c] += __shfl_xor_sync(full, v[c], o);
-  const unsigned act = __ballot_sync(full, active);
-  if (!active) return;
-  double fn[3];
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    x[c] = a.node_x0[3 * nd + c] + v[c] * a.dt;
-    fn[c] = -a.ibm_area_k * (x[c] - a.node_ref[3 * nd + c]);
-  }
-  if (sub == 0) {
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      a.node_x[3 * nd + c] = x[c];
-      a.node_x0[3 * nd + c] = x[c];
-      a.node_vel[3 * nd + c] = v[c];
-      a.node_force[3 * nd + c] = fn[c];
-    }
-  }
-  origin(x);
-  const int ii = lo[0] + di, jj = lo[1] + dj, kk = lo[2] + dk;
-  const long long cell = (long long)ii + (long long)jj * xc + (long long)kk * yc * xc;
-  int target = -1;
-  float f[3] = {0.f, 0.f, 0.f};
-  if (cell < a.C && cell >= 0) {
-    const double wgt = (1 - fabs(ii + 0.5 - r[0])) * (1 - fabs(jj + 0.5 - r[1])) *
-                       (1 - fabs(kk + 0.5 - r[2])) * a.ibm_inv_dx3 / U;
-    target = a.ibm_map[cell];
-#pragma unroll
-    for (int c = 0; c < 3; c++) f[c] = (float)(fn[c] * wgt);
-  }
-  spread_aggregated(act, target, f, a.fforce_x, a.fforce_y, a.fforce_z);
 }
 
 inline int blocks_for(long long n, int bs) { return (int)((n + bs - 1) / bs); }
 
 template <int RK>
-void launch_update32_rk(const KernelArgs& a, int nb, cudaStream_t s) {
+void launch_update32_rk(const KernelArgs& a, cudaStream_t s) {
+  const int nb = blocks_for(a.C, kBlock);
   if (a.K2 <= 4)
     k_update32<RK, 4><<<nb, kBlock, 0, s>>>(a);
   else if (a.K2 <= 6)
@@ -396,6 +347,11 @@ void launch_update32_rk(const KernelArgs& a, int nb, cudaStream_t s) {
 }
 
 }  // namespace
+
+void launch_record_sides32(const void* frec0, const void* frec1, int n, int32_t* out,
+                           cudaStream_t s) {
+  k_record_sides32<<<blocks_for(n, kBlock), kBlock, 0, s>>>(frec0, frec1, n, out);
+}
 
 void launch_gradient32(const KernelArgs& a, cudaStream_t s) {
   if (a.compact && a.wtab)
@@ -413,13 +369,12 @@ void launch_flux32(const KernelArgs& a, cudaStream_t s) {
                       0, s>>>(a);
 }
 void launch_update32(const KernelArgs& a, int rk, cudaStream_t s, bool finish) {
-  const int nb = blocks_for(a.C, kBlock);
   switch (rk) {
-    case 0: launch_update32_rk<0>(a, nb, s); break;
-    case 1: launch_update32_rk<1>(a, nb, s); break;
-    case 2: launch_update32_rk<2>(a, nb, s); break;
+    case 0: launch_update32_rk<0>(a, s); break;
+    case 1: launch_update32_rk<1>(a, s); break;
+    case 2: launch_update32_rk<2>(a, s); break;
     default:
-      launch_update32_rk<3>(a, nb, s);
+      launch_update32_rk<3>(a, s);
       if (finish) k_finish32<<<1, kFinishBlock, 0, s>>>(a);
       break;
   }

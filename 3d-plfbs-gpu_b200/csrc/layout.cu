@@ -761,6 +761,15 @@ int grid_for(long long n) {
 
 }  // namespace
 
+void launch_exclusive_scan(const int32_t* count, int n, int32_t* off, int32_t* wsum,
+                           int32_t* wbase, int32_t* info, cudaStream_t st) {
+  const int nwin = (n + kFaceWindow - 1) / kFaceWindow;
+  DevMesh m{};
+  m.C = n;
+  k_window_scan<<<nwin, kWinBlock, 0, st>>>(m, count, count, off, wsum, info);
+  k_window_base<<<1, kWinBlock, 0, st>>>(wsum, nwin, wbase);
+}
+
 void launch_polymesh_geometry(const DevPolyMesh& pm, double ref_dt, const GeometryOut& o,
                               const GeometryScratch& s, cudaStream_t st) {
   const int nwin = (pm.C + kFaceWindow - 1) / kFaceWindow;

@@ -285,6 +285,37 @@ struct DevStats {
   alignas(128) double history[kHistoryCap][6];
 };
 
+// Tables of the march kernel (march.cu), built by tiles.cu: n tiles of T
+// cells (the last one shorter) along a space-filling curve. Per tile, SC rows
+// of local cells (own cells, then halo cells, then -1) and SF faces:
+//   cell [n][SC]     device cell of each local cell
+//   nbr  [n][K][SC]  its stencil neighbours (st_nbr's entries)
+//   wset [n][SC]     its weight set (compact layout, else null)
+//   ij   [n][SF]     local owner | local neighbour << 11 (kTileGhost: boundary
+//                    face) | low 10 branch bits << 22
+//   fid  [n][SF]     device face | high 4 branch bits << 28
+//   rec  [n][SF]     its unique record (compact layout, else null)
+//   slot [n][K2][T]  own cells' faces in gather order: local face << 1 | (cell
+//                    is the neighbour), 0xffff in empty slots
+//   count [n]        (local cells, faces)
+constexpr int kTileGhost = 2047;
+constexpr int kTileMaxCells = 2046;  // local indices fit 11 bits
+constexpr int kTileMaxFaces = 4096;
+struct TileArgs {
+  int n, T, SC, SF;
+  int smem;  // dynamic shared memory of a block
+  int tables;  // 1: the compact tables are copied there
+  int place;   // the tile's tables there: 1 slot, 2 ij and rec / fid, 4 cell, nbr, wset
+  int32_t* cell;
+  int32_t* nbr;
+  int32_t* wset;
+  uint32_t* ij;
+  int32_t* fid;
+  int32_t* rec;
+  uint16_t* slot;
+  int2* count;
+};
+
 // Tensor maps of the FP64 state and gradient rows for the TMA-staged flux
 // kernel (k_flux_tma): 2D, one cell per row, boxes one row high.
 struct FluxMaps {
@@ -313,6 +344,7 @@ struct KernelArgs {
   double rho0, uref;
   // arrays (FP64 path)
   void* state;          // double4 [C+B]
+  void* state2;         // double4 [C+B]: the march kernel's other state array
   void* t0;             // double4 [C]
   void* t1;             // double4 [C]
   void* grad;           // 3 x double4 per cell [3C]
@@ -345,9 +377,17 @@ struct KernelArgs {
   const void* frec0; const void* frec1; const void* frec2;  // double4 (FP32: float4) [unique]
   const int32_t* cell_wset;                       // [C] index into wtab
   const void* wtab;                               // [unique sets][K][3] double (FP32: float)
-  const int32_t* frec_sides;                      // [unique records] branch bits (FP64)
+  int n_frec, n_wset;                             // unique records and weight sets
+  const int32_t* frec_sides;                      // [unique records] branch bits
   const double* frec_relax;                       // [2 x unique records] (1 - tau) A cd, tau A cd (FP64)
   int compact;                                    // 1: the kernels read the tables
+  // Residual sums of a context that marches: in the last stage cells are taken
+  // along red_order, every 32 of them give a partial sum and red_warps of those
+  // a tile's, as the march kernel adds them (null: blocks in cell order)
+  const int32_t* red_order;
+  int red_warps;
+  TileArgs tiles;                                 // n = 0: no march kernel
+  unsigned* grid_bar;                             // its barrier counter
 };
 
 // Launchers (kernels.cu; the FP32 deviation form in kernels_fp32.cu). All
@@ -364,6 +404,49 @@ void launch_update(const KernelArgs& a, int precision, int rk, cudaStream_t stre
                    bool finish = true);
 void launch_finish(const KernelArgs& a, int precision, cudaStream_t stream);
 void launch_seed(const KernelArgs& a, int precision, bool conserved, cudaStream_t stream);
+// The march kernel (march.cu): nsteps time steps in one cooperative launch,
+// up to the step that halts the context. march_smem: a block's dynamic shared
+// memory for t's T, SC and SF within `most` bytes (0: none), and where t's
+// tables go (t.tables, t.place).
+cudaError_t launch_march(const KernelArgs& a, int precision, int nsteps, cudaStream_t stream);
+int march_max_own();
+int march_max_tiles();
+int march_smem(const KernelArgs& a, int precision, int most, TileArgs& t);
+
+// Exclusive scan of n ints in two levels (layout.cu): item i's prefix is
+// wbase[i / kFaceWindow] + off[i]; wsum and wbase hold one int per window (and
+// one more), info two ints of scratch.
+void launch_exclusive_scan(const int32_t* count, int n, int32_t* off, int32_t* wsum,
+                           int32_t* wbase, int32_t* info, cudaStream_t stream);
+
+// The cells along a Hilbert curve through their centroids (tiles.cu), device
+// numbering.
+struct CurveScratch {
+  double* part;       // [CurveSizes::part]
+  uint32_t* key[2];   // [C]
+  int32_t* val[2];    // [C]
+  int32_t* count;     // [CurveSizes::count]
+  int32_t* off;       // [CurveSizes::count]
+  int32_t* wsum;      // [CurveSizes::windows]
+  int32_t* wbase;     // [CurveSizes::windows + 1]
+  int32_t* info;      // [4]
+};
+struct CurveSizes {
+  size_t part, count, windows;
+};
+CurveSizes curve_sizes(int C);
+void launch_cell_curve(const DevMesh& m, const CurveScratch& s, int32_t* order,
+                       cudaStream_t stream);
+// Cut into tiles of T cells, each sorted by device index, and the inverse.
+void launch_tile_order(int C, int T, int32_t* order, int32_t* pos, cudaStream_t stream);
+// The tile tables: branch bits of all faces, the largest tile's faces and cut
+// faces (most[2], zeroed), and the tables themselves.
+void launch_face_sides(const KernelArgs& a, int precision, uint16_t* side, cudaStream_t stream);
+void launch_tile_count(const KernelArgs& a, const int32_t* order, const int32_t* pos, int T,
+                       int32_t* most, cudaStream_t stream);
+void launch_tile_build(const KernelArgs& a, const int32_t* order, const int32_t* pos,
+                       const uint16_t* side, const TileArgs& t, int max_faces, int max_cut,
+                       cudaStream_t stream);
 void launch_wall_forces(const KernelArgs& a, int precision, const int* walls, int n,
                         double visc_gamma, double gamma, double* out, cudaStream_t stream);
 void launch_ibm32(const KernelArgs& a, cudaStream_t stream);
@@ -372,6 +455,8 @@ void launch_ibm32(const KernelArgs& a, cudaStream_t stream);
 // relax[2r] = (1 - tau) A cd, relax[2r + 1] = tau A cd (cd = KernelArgs::eq_cd).
 void launch_record_sides(const void* frec0, const void* frec1, const void* frec2, double cd, int n,
                          int flavour, int32_t* out, double* relax, cudaStream_t stream);
+void launch_record_sides32(const void* frec0, const void* frec1, int n, int32_t* out,
+                           cudaStream_t stream);
 void launch_gradient32(const KernelArgs& a, cudaStream_t stream);
 void launch_flux32(const KernelArgs& a, cudaStream_t stream);
 void launch_update32(const KernelArgs& a, int rk, cudaStream_t stream, bool finish = true);

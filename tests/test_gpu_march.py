@@ -1,0 +1,116 @@
+"""The march kernel (plfbs_run on a mesh that fits one tile per SM) against the
+same RK stages run one kernel at a time (plfbs_run_stages): the arithmetic and
+the order of every sum are the same, so states, residual records, gradients and
+fluxes agree bit for bit, over cell counts at the edges of the tiles, both
+precisions and flavours, with and without the compact layout, and where the
+context halts in the middle of a march."""
+
+import numpy as np
+import pytest
+
+from plfbs import capi, cases
+
+pytestmark = pytest.mark.gpu
+
+STEPS = 5
+
+
+def _mesh(kind, n):
+    sides = ["inlet", "outlet", "side", "side", "side", "side"]
+    if kind == "tets":
+        pm = cases.jittered_tet_box(n[0], jitter=0.1, seed=3, patch_types=["side"] * 6)
+    elif kind == "graded":
+        grid = [np.concatenate([[0.0], np.cumsum(1.03 ** np.arange(k))]) for k in n]
+        pm = cases.hex_box(*grid, patch_types=sides)
+    else:
+        pm = cases.uniform_box(*n, patch_types=sides)
+    c = cases.Case(mesh_dir="", X=n[0], Y=n[1], Z=n[2], dt=0.05, mach=0.05, reynolds=50.0,
+                   ref_length=4.0,
+                   bcs=[cases.BC("inlet", 1, 1, 0, 0, "dirichlet", "neumann"),
+                        cases.BC("outlet", 1, 0, 0, 0, "neumann", "dirichlet"),
+                        cases.BC("side", 1, 0, 0, 0, "dirichlet", "neumann")])
+    return cases.mesh_arrays(pm, c.visc, c.gamma, c.fneq_min), c
+
+
+def _solver(ma, c, precision, flavour, renumber, tolerance=0.0):
+    rt, vt, val = cases.bc_arrays(ma, c)
+    cfg = dict(visc=c.visc, dt=c.dt, max_velocity=c.mach, channel_height=c.Y,
+               lengths=(c.X, c.Y, c.Z), renumber=renumber, flavour=flavour, precision=precision,
+               pressure_gradient=1e-5, tolerance=tolerance,
+               gradient_mode=capi.GRAD_LS | capi.GRAD_EXACT_INVERSE)
+    return capi.Solver(ma, rt, vt, val, cfg)
+
+
+def _start(ma):
+    rng = np.random.default_rng(2)
+    q = np.zeros((ma.total_cells, 4))
+    q[:, 0] = 0.04 + 0.002 * rng.standard_normal(ma.total_cells)
+    q[:, 1:3] = 0.002 * rng.standard_normal((ma.total_cells, 2))
+    q[:, 3] = 1.0 + 0.001 * rng.standard_normal(ma.total_cells)
+    return q
+
+
+def _same(ma, c, precision, flavour, renumber, compress=None):
+    out = []
+    for march in (True, False):
+        s = _solver(ma, c, precision, flavour, renumber)
+        if compress is not None:
+            s.set_layout_compression(compress)
+        s.set_state(_start(ma))
+        if march:
+            _, h = s.run(STEPS)
+        else:
+            s.run_stages(4 * STEPS)
+            h = None
+        grad, flux, state = s.gradients(), s.face_flux(), s.get_state()
+        _, h2 = s.run(1)  # carries on from either
+        out.append((grad, flux, state, h2, s.get_state()))
+        s.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    assert np.isfinite(out[0][2]).all()
+
+
+# 1 cell; one tile of 32 and one cell more; one tile per SM of 32 and one cell
+# more (148 SMs); several rounds of faces per block; a ragged last tile
+@pytest.mark.parametrize("n", [(1, 1, 1), (8, 4, 1), (11, 3, 1), (37, 16, 8), (421, 9, 1),
+                               (41, 29, 23), (40, 40, 41)])
+@pytest.mark.parametrize("precision", [capi.FP64, capi.FP32_DEVIATION])
+def test_march_is_the_stages_boxes(plfbs_lib, n, precision):
+    ma, c = _mesh("box", n)
+    _same(ma, c, precision, capi.FLAVOUR_GPU, 0)
+
+
+@pytest.mark.parametrize("kind,n", [("tets", (2, 2, 2)), ("tets", (11, 11, 11)),
+                                    ("graded", (13, 11, 9)), ("box", (24, 20, 18))])
+@pytest.mark.parametrize("precision,flavour", [(capi.FP64, capi.FLAVOUR_GPU),
+                                               (capi.FP64, capi.FLAVOUR_CPU_SOLVER),
+                                               (capi.FP32_DEVIATION, capi.FLAVOUR_GPU)])
+@pytest.mark.parametrize("renumber", [0, 1])
+def test_march_is_the_stages(plfbs_lib, kind, n, precision, flavour, renumber):
+    ma, c = _mesh(kind, n)
+    _same(ma, c, precision, flavour, renumber, 0 if kind == "box" else None)
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.FP32_DEVIATION])
+def test_march_halts_at_the_step(plfbs_lib, precision):
+    """A tolerance that the residual passes after a few steps: the march stops
+    with that step's state, and a march of one step at a time does the same."""
+    ma, c = _mesh("box", (12, 10, 9))
+    s = _solver(ma, c, precision, capi.FLAVOUR_GPU, 0)
+    s.set_state(_start(ma))
+    _, h = s.run(40)
+    tol = float(h[17:20, 1].min())
+    assert (h[:17, 1] > tol).all()
+    first = int(np.argmax(h[:, 1] < np.nextafter(tol, 1)))
+    s.close()
+    out = []
+    for chunk in (40, 1):
+        s = _solver(ma, c, precision, capi.FLAVOUR_GPU, 0, tolerance=np.nextafter(tol, 1))
+        s.set_state(_start(ma))
+        for _ in range(40 // chunk):
+            st, _ = s.run(chunk)
+        assert st["converged"] and st["steps_done"] == first + 1
+        out.append(s.get_state())
+        s.close()
+    np.testing.assert_array_equal(out[0], out[1])
