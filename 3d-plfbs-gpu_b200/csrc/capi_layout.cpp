@@ -507,7 +507,7 @@ int build_compact_layout(plfbs_ctx* ctx) {
       ctx->compact_faces = a.n_frec = U;
       TRY(pool_alloc(ctx, &p, 4 * (size_t)U));
       if (fp32) {
-        plfbs::launch_record_sides32(t[0], t[1], U, static_cast<int32_t*>(p), ctx->stream);
+        plfbs::launch_record_sides32(t[0], t[1], t[2], U, static_cast<int32_t*>(p), ctx->stream);
         a.frec_sides = static_cast<const int32_t*>(p);
       } else {
         void* relax = nullptr;

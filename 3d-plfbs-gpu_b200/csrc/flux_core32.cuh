@@ -10,6 +10,7 @@
 
 #include <cstdint>
 
+#include "flux_core.cuh"
 #include "plfbs_internal.hpp"
 
 namespace plfbs {
@@ -274,6 +275,54 @@ __device__ __forceinline__ void boundary_sides32(const KernelArgs& a, const int 
   }
 #pragma unroll
   for (int k = 0; k < 12; k++) g1[k] = g2[k];
+}
+
+// Records of faces along a coordinate axis, as face_kind and axis_flux in
+// flux_core.cuh.
+__device__ __forceinline__ unsigned face_kind32(const f4& f0, const f4& f1, const f4& f2,
+                                                unsigned sides) {
+  const float n[3] = {f0.x, f0.y, f0.z}, t1[3] = {f1.y, f1.z, f1.w}, t2[3] = {f2.x, f2.y, f2.z};
+  const unsigned want[3] = {axis_sides<0, 0>(), axis_sides<0, 1>(), axis_sides<0, 2>()};
+  for (int x = 0; x < 3; x++) {
+    bool ok = sides == want[x];
+    for (int c = 0; c < 3; c++)
+      if (c != x) ok = ok && n[c] == 0.0f && t1[c] == 0.0f && t2[c] == 0.0f;
+    if (ok) return 1u + x;
+  }
+  return 0u;
+}
+
+template <int AX>
+__device__ __forceinline__ f4 axis_flux32(const KernelArgs& a, const float dt, const float t1d,
+                                          const float t2d, const float nd, const float area,
+                                          const float tau, const f4& qo, const f4& qn,
+                                          float g1[12], float g2[12]) {
+  const float qov[4] = {qo.w, qo.x, qo.y, qo.z}, qnv[4] = {qn.w, qn.x, qn.y, qn.z};
+  float si[4], sn[4], sc[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    si[k] = __fadd_rn(qov[k], -__fmul_rn(t1d, g1[3 * k + AX]));
+    sn[k] = __fadd_rn(qnv[k], -__fmul_rn(t2d, g2[3 * k + AX]));
+    sc[k] = __fmul_rn(__fadd_rn(si[k], sn[k]), 0.5f);
+  }
+  const Eq32 k{a.eq32_k0, a.eq32_k1, a.rho0f};
+  float R, m[3], P[6];
+  face_moments32(k, dt, axis_sides<0, AX>(), si, sn, sc, g1, g2, R, m, P);
+  const float mn = __fmul_rn(m[AX], nd);
+  constexpr int C0 = AX == 0 ? 0 : AX == 1 ? 3 : 4, C1 = AX == 0 ? 3 : AX == 1 ? 1 : 5,
+                C2 = AX == 0 ? 4 : AX == 1 ? 5 : 2;
+  const float Pn[3] = {__fmul_rn(P[C0], nd), __fmul_rn(P[C1], nd), __fmul_rn(P[C2], nd)};
+  const float cA = __fmul_rn(area, a.eq32_cd), sA = __fmul_rn(cA, a.inv_uref_f);
+  const float omA = __fmul_rn(__fadd_rn(1.0f, -tau), sA), tA = __fmul_rn(tau, sA);
+  const float mnr = __fdiv_rn(__fmul_rn(mn, a.eq32_pgcd), fmaf(a.eq32_cd, R, k.rho0));
+  const float al = __fmul_rn(omA, mnr), be = __fmul_rn(omA, __fmul_rn(R, 1.0f / 3.0f));
+  float out[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const float tp = __fmul_rn(tA, Pn[c]);
+    out[c] = fmaf(al, m[c], c == AX ? fmaf(be, nd, tp) : tp);
+  }
+  return f4{out[0], out[1], out[2], __fmul_rn(mn, cA)};
 }
 
 // The face flux in deviation form: the rho0 / 3 n A part of the momentum flux

@@ -123,21 +123,33 @@ __device__ __forceinline__ void flux_face(const KernelArgs& a, const int f, cons
            f2 = ld4(CR ? a.frec2 : a.face2, r);
   const int o = ids.x, nb = ids.y;
   const double dt = f1.x;
-  const double t1[3] = {f1.y, f1.z, f1.w}, t2[3] = {f2.x, f2.y, f2.z};
+  // the branch decisions: per record with the compact layout (FP64 compact
+  // layouts always carry them)
+  unsigned sides = CR ? (unsigned)__ldg(a.frec_sides + r) : 0u;
   const d4 qo = ld4(a.state, o);
   double g1[12], g2[12], si[4], sn[4], sc[4];
   load_grad(a.grad, o, g1);
+  const double t1[3] = {f1.y, f1.z, f1.w}, t2[3] = {f2.x, f2.y, f2.z};
   if (nb < a.C) {
     const d4 qn = ld4(a.state, nb);
     load_grad(a.grad, nb, g2);
+    if (CR && (sides >> kKindShift)) {
+      const double2 w = __ldg(reinterpret_cast<const double2*>(a.frec_relax) + r);
+      const double cA = __dmul_rn(f0.w, a.eq_cd);
+      const unsigned kind = sides >> kKindShift;
+      const d4 x =
+          kind == 1 ? axis_flux<FL, 0>(a, dt, t1[0], t2[0], f0.x, cA, w.x, w.y, qo, qn, g1, g2)
+          : kind == 2 ? axis_flux<FL, 1>(a, dt, t1[1], t2[1], f0.y, cA, w.x, w.y, qo, qn, g1, g2)
+                      : axis_flux<FL, 2>(a, dt, t1[2], t2[2], f0.z, cA, w.x, w.y, qo, qn, g1, g2);
+      st4(a.flux, f, x);
+      return;
+    }
     interior_sides(t1, t2, qo, qn, g1, g2, si, sn, sc);
   } else {
     boundary_sides<FL>(a, nb - a.C, t1, t2, qo, g1, g2, si, sn, sc);
   }
-  // the branch decisions: per record with the compact layout (FP64 compact
-  // layouts always carry them)
   const double n[3] = {f0.x, f0.y, f0.z};
-  const unsigned sides = CR ? (unsigned)__ldg(a.frec_sides + r) : face_sides<FL>(n, dt);
+  if (!CR) sides = face_sides<FL>(n, dt);
   st4(a.flux, f, face_flux<FL, CR>(a, r, sides, dt, si, sn, sc, g1, g2));
 }
 
@@ -616,7 +628,8 @@ __global__ void k_record_sides(const void* frec0, const void* frec1, const void*
     const double cA = __dmul_rn(f0.w, cd);
     relax[r] = make_double2(__dmul_rn(__dadd_rn(1.0, -f2.w), cA), __dmul_rn(f2.w, cA));
     const double nv[3] = {f0.x, f0.y, f0.z};
-    out[r] = (int32_t)face_sides<FL>(nv, f1.x);
+    const unsigned sides = face_sides<FL>(nv, f1.x);
+    out[r] = (int32_t)(sides | face_kind<FL>(f0, f1, f2, sides) << kKindShift);
   }
 }
 

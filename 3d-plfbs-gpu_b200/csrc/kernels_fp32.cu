@@ -108,14 +108,24 @@ __device__ __forceinline__ void flux_face32(const KernelArgs& a, const int f, co
   const f4 qo = ldf(a.state, o);
   float g1[12], g2[12], si[4], sn[4], sc[4];
   load_grad32(a.grad, o, g1);
+  unsigned sides = CR ? (unsigned)__ldg(a.frec_sides + rec) : 0u;
   if (nb < a.C) {
     const f4 qn = ldf(a.state, nb);
     load_grad32(a.grad, nb, g2);
+    if (CR && (sides >> kKindShift)) {
+      const unsigned kind = sides >> kKindShift;
+      const f4 x =
+          kind == 1 ? axis_flux32<0>(a, dt, t1[0], t2[0], n[0], f0.w, f2.w, qo, qn, g1, g2)
+          : kind == 2 ? axis_flux32<1>(a, dt, t1[1], t2[1], n[1], f0.w, f2.w, qo, qn, g1, g2)
+                      : axis_flux32<2>(a, dt, t1[2], t2[2], n[2], f0.w, f2.w, qo, qn, g1, g2);
+      stf(a.flux, f, x);
+      return;
+    }
     interior_sides32(t1, t2, qo, qn, g1, g2, si, sn, sc);
   } else {
     boundary_sides32(a, nb - a.C, t1, t2, qo, g1, g2, si, sn, sc);
   }
-  const unsigned sides = face_sides32(n[0], n[1], n[2], __fmul_rn(0.001f, dt));
+  if (!CR) sides = face_sides32(n[0], n[1], n[2], __fmul_rn(0.001f, dt));
   stf(a.flux, f, face_flux32(a, n, f0.w, f2.w, sides, dt, si, sn, sc, g1, g2));
 }
 
@@ -324,10 +334,12 @@ __global__ void __launch_bounds__(kIbmBlock) k_ibm32(const KernelArgs a) {
 }
 
 // Branch bits of the compact layout's unique records.
-__global__ void k_record_sides32(const void* frec0, const void* frec1, int n, int32_t* out) {
+__global__ void k_record_sides32(const void* frec0, const void* frec1, const void* frec2, int n,
+                                 int32_t* out) {
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    const f4 f0 = ldf(frec0, r);
-    out[r] = (int32_t)face_sides32(f0.x, f0.y, f0.z, __fmul_rn(0.001f, ldf(frec1, r).x));
+    const f4 f0 = ldf(frec0, r), f1 = ldf(frec1, r);
+    const unsigned sides = face_sides32(f0.x, f0.y, f0.z, __fmul_rn(0.001f, f1.x));
+    out[r] = (int32_t)(sides | face_kind32(f0, f1, ldf(frec2, r), sides) << kKindShift);
   }
 }
 
@@ -348,9 +360,9 @@ void launch_update32_rk(const KernelArgs& a, cudaStream_t s) {
 
 }  // namespace
 
-void launch_record_sides32(const void* frec0, const void* frec1, int n, int32_t* out,
-                           cudaStream_t s) {
-  k_record_sides32<<<blocks_for(n, kBlock), kBlock, 0, s>>>(frec0, frec1, n, out);
+void launch_record_sides32(const void* frec0, const void* frec1, const void* frec2, int n,
+                           int32_t* out, cudaStream_t s) {
+  k_record_sides32<<<blocks_for(n, kBlock), kBlock, 0, s>>>(frec0, frec1, frec2, n, out);
 }
 
 void launch_gradient32(const KernelArgs& a, cudaStream_t s) {

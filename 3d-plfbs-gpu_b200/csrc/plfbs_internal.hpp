@@ -378,7 +378,7 @@ struct KernelArgs {
   const int32_t* cell_wset;                       // [C] index into wtab
   const void* wtab;                               // [unique sets][K][3] double (FP32: float)
   int n_frec, n_wset;                             // unique records and weight sets
-  const int32_t* frec_sides;                      // [unique records] branch bits
+  const int32_t* frec_sides;                      // [unique records] branch bits and kind
   const double* frec_relax;                       // [2 x unique records] (1 - tau) A cd, tau A cd (FP64)
   int compact;                                    // 1: the kernels read the tables
   // Residual sums of a context that marches: in the last stage cells are taken
@@ -455,8 +455,8 @@ void launch_ibm32(const KernelArgs& a, cudaStream_t stream);
 // relax[2r] = (1 - tau) A cd, relax[2r + 1] = tau A cd (cd = KernelArgs::eq_cd).
 void launch_record_sides(const void* frec0, const void* frec1, const void* frec2, double cd, int n,
                          int flavour, int32_t* out, double* relax, cudaStream_t stream);
-void launch_record_sides32(const void* frec0, const void* frec1, int n, int32_t* out,
-                           cudaStream_t stream);
+void launch_record_sides32(const void* frec0, const void* frec1, const void* frec2, int n,
+                           int32_t* out, cudaStream_t stream);
 void launch_gradient32(const KernelArgs& a, cudaStream_t stream);
 void launch_flux32(const KernelArgs& a, cudaStream_t stream);
 void launch_update32(const KernelArgs& a, int rk, cudaStream_t stream, bool finish = true);
