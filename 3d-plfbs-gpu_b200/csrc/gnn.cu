@@ -231,6 +231,8 @@ struct Fwd {
   const float* b1;  // [64]
   const bf16* W2;   // [64][NOUT]
   const float* b2;  // [NOUT]
+  const bf16* W1t;  // tcgen05: W1 and W2 transposed, in the canonical layout
+  const bf16* W2t;
   float* z1;        // [M][64] pre-activations, or null (inference)
   float* y;         // [M][NOUT]
 };
@@ -409,77 +411,113 @@ __device__ __forceinline__ void stg8(float* p, const float* v) {
                : "memory");
 }
 
-// As load_x, into the canonical layout. Thread t takes row t % 128 of the tile
-// and its 8-element (16-byte) chunks t / 128, t / 128 + 2, ...: a warp's stores
-// fill whole core matrices (no bank conflicts) and each thread reads whole
-// 32-byte sectors. The row's sources (its node rows for an edge MLP, its CSR
-// range for a node MLP) are read once, and the chunks are loaded four at a
-// time, so that a thread has four independent gathers in flight rather than
-// one (the kernels are bound by the latency of these gathers); a group of
-// four chunks covers one 64-column input segment.
+// As load_x, into the canonical layout. A lane takes one 8-element (32-byte)
+// chunk: lanes l and l + 8 k of a warp the same row, chunk k of a 128-byte line
+// (ENC, whose rows are two chunks: 16 rows of two), so that a warp's load touches
+// eight whole lines (one line per lane, as with a row per thread, was bound by
+// L1's tag lookups) and eight lanes' stores fill one core matrix (no bank
+// conflicts). Warp w takes rows 8w .. 8w + 7 and the same 64 rows on. The loads
+// of a row (its six lines for an edge MLP, two for a node MLP and then two lines
+// of up to six edges, hexahedra having six) are all in flight together.
+constexpr int kAggEdges = 6;
+__device__ __forceinline__ void put_chunk(unsigned char* As, int r, int c, int K1,
+                                          const float (&v)[8]) {
+  __nv_bfloat162 b[4] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3]),
+                         __floats2bfloat162_rn(v[4], v[5]), __floats2bfloat162_rn(v[6], v[7])};
+  *reinterpret_cast<uint4*>(As + canon_off(r, 8 * c, K1)) = *reinterpret_cast<const uint4*>(b);
+}
 template <int MODE, int K1>
 __device__ __forceinline__ void load_x_canon(const Rows& a, int row0, unsigned char* As) {
-  constexpr int C8 = K1 / 8, NQ = TM * C8 / kTcThreads, G = NQ < 4 ? NQ : 4;
-  static_assert(kTcThreads == 2 * TM && (TM * C8) % kTcThreads == 0 && NQ % G == 0,
-                "chunks per thread");
-  const int r = threadIdx.x % TM, kc0 = threadIdx.x / TM, m = row0 + r;
-  const bool valid = m < a.M;
-  const float *p0 = nullptr, *p1 = nullptr, *p2 = nullptr;
-  int e0 = 0, e1 = 0;
-  if (valid) {
-    p0 = a.x0 + (size_t)m * (MODE == ENC ? FP : H);
-    if (MODE == EDGE) {
-      p1 = a.hs + (size_t)a.src[m] * H;
-      p2 = a.hs + (size_t)a.dst[m] * H;
+  static_assert(kTcThreads == 256 && TM == 128 && (K1 == FP || K1 % 32 == 0), "row groups");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (MODE == ENC) {
+    const int r = 16 * warp + (lane & 15), c = lane >> 4, m = row0 + r;
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (m < a.M) ldg8(a.x0 + (size_t)m * FP + 8 * c, v);
+    put_chunk(As, r, c, K1, v);
+    return;
+  }
+  const int c0 = lane >> 3;  // chunk within a line
+  // lines of plain rows: the own row and, for an edge MLP, its two nodes'
+  constexpr int NL = MODE == EDGE ? 6 : 2;
+#pragma unroll 1
+  for (int half = 0; half < 2; half++) {
+    const int r = 64 * half + 8 * warp + (lane & 7), m = row0 + r;
+    const bool valid = m < a.M;
+    const float *p0 = nullptr, *p1 = nullptr, *p2 = nullptr;
+    int e0 = 0, e1 = 0;
+    if (valid) {
+      p0 = a.x0 + (size_t)m * H;
+      if (MODE == EDGE) {
+        p1 = a.hs + (size_t)a.src[m] * H;
+        p2 = a.hs + (size_t)a.dst[m] * H;
+      }
+      if (MODE == NODE) {
+        e0 = a.in_off[m];
+        e1 = a.in_off[m + 1];
+      }
+    }
+    int edge[kAggEdges];
+    if (MODE == NODE) {
+#pragma unroll
+      for (int k = 0; k < kAggEdges; k++) edge[k] = e0 + k < e1 ? __ldg(a.in_idx + e0 + k) : -1;
+    }
+    float v[NL][8];
+#pragma unroll
+    for (int g = 0; g < NL; g++) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) v[g][j] = 0.f;
+      const float* p = g < 2 ? p0 : (g < 4 ? p1 : p2);
+      if (valid) ldg8(p + 32 * (g & 1) + 8 * c0, v[g]);
     }
     if (MODE == NODE) {
-      e0 = a.in_off[m];
-      e1 = a.in_off[m + 1];
-    }
-  }
-#pragma unroll
-  for (int g0 = 0; g0 < NQ; g0 += G) {
-    float v[G][8];
-#pragma unroll
-    for (int i = 0; i < G; i++) {
-      const int c = kc0 + 2 * (g0 + i);  // this chunk: columns 8c .. 8c + 7
-#pragma unroll
-      for (int j = 0; j < 8; j++) v[i][j] = 0.f;
-      if (valid && !(MODE == NODE && c >= 8)) {
-        const int seg = MODE == ENC ? 0 : c / 8;
-        const float* p = seg == 0 ? p0 : (seg == 1 ? p1 : p2);
-        ldg8(p + (MODE == ENC ? 8 * c : 8 * (c % 8)), v[i]);
-      }
-    }
-    if (MODE == NODE && kc0 + 2 * g0 >= 8) {
       // the aggregate segment: the sum of the edge states over the incoming
       // edges, in CSR order
-#pragma unroll 2
-      for (int e = e0; e < e1; e++) {
-        const float* pe = a.eagg + (size_t)a.in_idx[e] * H;
+      float u[kAggEdges][2][8];
 #pragma unroll
-        for (int i = 0; i < G; i++) {
-          float u[8];
-          ldg8(pe + 8 * (kc0 + 2 * (g0 + i) - 8), u);
+      for (int k = 0; k < kAggEdges; k++)
+        if (edge[k] >= 0) {
 #pragma unroll
-          for (int j = 0; j < 8; j++) v[i][j] += u[j];
+          for (int g = 0; g < 2; g++)
+            ldg8(a.eagg + (size_t)edge[k] * H + 32 * g + 8 * c0, u[k][g]);
         }
-      }
-    }
 #pragma unroll
-    for (int i = 0; i < G; i++) {
-      const int c = kc0 + 2 * (g0 + i);
-      __nv_bfloat162 b[4] = {
-          __floats2bfloat162_rn(v[i][0], v[i][1]), __floats2bfloat162_rn(v[i][2], v[i][3]),
-          __floats2bfloat162_rn(v[i][4], v[i][5]), __floats2bfloat162_rn(v[i][6], v[i][7])};
-      *reinterpret_cast<uint4*>(As + canon_off(r, 8 * c, K1)) =
-          *reinterpret_cast<const uint4*>(b);
+      for (int g = 0; g < NL; g++) put_chunk(As, r, 4 * g + c0, K1, v[g]);
+#pragma unroll
+      for (int g = 0; g < 2; g++) {
+        float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < kAggEdges; k++)
+          if (edge[k] >= 0)
+#pragma unroll
+            for (int j = 0; j < 8; j++) s[j] += u[k][g][j];
+        for (int e = e0 + kAggEdges; e < e1; e++) {
+          float w[8];
+          ldg8(a.eagg + (size_t)a.in_idx[e] * H + 32 * g + 8 * c0, w);
+#pragma unroll
+          for (int j = 0; j < 8; j++) s[j] += w[j];
+        }
+        put_chunk(As, r, 8 + 4 * g + c0, K1, s);
+      }
+    } else {
+#pragma unroll
+      for (int g = 0; g < NL; g++) put_chunk(As, r, 4 * g + c0, K1, v[g]);
     }
   }
 }
 
+// N 16-byte words into shared memory. The weights come as images of the layout
+// they have there (k_pack): placing them element by element took a block 12 to 18
+// thousand cycles, a tenth of the kernel.
+template <int N>
+__device__ __forceinline__ void copy16(unsigned char* dst, const bf16* src) {
+#pragma unroll 8
+  for (int i = threadIdx.x; i < N; i += kTcThreads)
+    reinterpret_cast<uint4*>(dst)[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
+}
+
 template <int MODE, int K1, int NOUT>
-__global__ void __launch_bounds__(kTcThreads) k_mlp_fwd_tc(const Fwd a, int* err) {
+__global__ void __launch_bounds__(kTcThreads, 2) k_mlp_fwd_tc(const Fwd a, int* err) {
   extern __shared__ __align__(16) unsigned char smem[];
   unsigned char* As = smem;                       // [128][K1]
   unsigned char* Hs = As + TM * K1 * 2;           // [128][64]
@@ -488,10 +526,8 @@ __global__ void __launch_bounds__(kTcThreads) k_mlp_fwd_tc(const Fwd a, int* err
   uint64_t* mbar = reinterpret_cast<uint64_t*>(W2t + NOUT * H * 2);
   uint32_t* slot = reinterpret_cast<uint32_t*>(mbar + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < K1 * H; i += kTcThreads)
-    *reinterpret_cast<bf16*>(W1t + canon_off(i % H, i / H, K1)) = a.W1[i];
-  for (int i = tid; i < H * NOUT; i += kTcThreads)
-    *reinterpret_cast<bf16*>(W2t + canon_off(i % NOUT, i / NOUT, H)) = a.W2[i];
+  copy16<K1 * H / 8>(W1t, a.W1t);
+  copy16<H * NOUT / 8>(W2t, a.W2t);
   if (tid == 0) mbar_init(mbar, 1);
   if (warp == 0) tmem_alloc(slot, 128);
   fence_async_smem();
@@ -519,6 +555,14 @@ __global__ void __launch_bounds__(kTcThreads) k_mlp_fwd_tc(const Fwd a, int* err
       umma_commit(mbar);
     }
     __syncwarp();
+    // the residual (the row's own previous state) is on its way before the waits
+    constexpr bool kRes = MODE == EDGE || MODE == NODE;
+    float res[kRes ? 4 : 1][8];
+    if (kRes && m < a.x.M) {
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        ldg8(a.x.x0 + (size_t)m * H + 32 * half + 8 * k, res[kRes ? k : 0]);
+    }
     ok = mbar_wait(mbar, parity);
     parity ^= 1u;
     tc_fence_after();
@@ -560,14 +604,12 @@ __global__ void __launch_bounds__(kTcThreads) k_mlp_fwd_tc(const Fwd a, int* err
       float v[16];
       tmem_ld16(d2 + lanes + c0, v);
       if (m < a.x.M) {
-        if (MODE == EDGE || MODE == NODE) {  // residual: the row's own previous state
-          float p0[8], p1[8];
-          ldg8(a.x.x0 + (size_t)m * H + c0, p0);
-          ldg8(a.x.x0 + (size_t)m * H + c0 + 8, p1);
+        if (kRes) {
+          const int k = (c0 - 32 * half) / 8;
 #pragma unroll
           for (int i = 0; i < 8; i++) {
-            v[i] += p0[i];
-            v[8 + i] += p1[i];
+            v[i] += res[kRes ? k : 0][i];
+            v[8 + i] += res[kRes ? k + 1 : 0][i];
           }
         }
 #pragma unroll
@@ -603,6 +645,8 @@ struct Bwd {
   const float* z1;    // [M][64]
   const bf16* W1;
   const bf16* W2;
+  const bf16* W1c;  // tcgen05: the same in the canonical layout
+  const bf16* W2c;
   float* dx0;    // EDGE/NODE: dy + dX1[:, 0:64]; DEC: dX1 ([M][64]); ENC: unused
   float* dseg1;  // EDGE: dX1[:, 64:128] per edge (to src); NODE: dX1[:, 64:128] (aggregate)
   float* dseg2;  // EDGE: dX1[:, 128:192] per edge (to dst)
@@ -814,10 +858,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_bwd_tc(const Bwd a, int* 
   static_assert(NOUT % 16 == 0 && K1 % 16 == 0, "MMA shapes");
   constexpr int GB2 = (TM * (NOUT / 8) + kTcThreads - 1) / kTcThreads * 8;  // dY columns a thread sums
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < K1 * H; i += kTcThreads)
-    *reinterpret_cast<bf16*>(W1c + canon_off(i / H, i % H, H)) = a.W1[i];
-  for (int i = tid; i < H * NOUT; i += kTcThreads)
-    *reinterpret_cast<bf16*>(W2c + canon_off(i / NOUT, i % NOUT, NOUT)) = a.W2[i];
+  copy16<K1 * H / 8>(W1c, a.W1c);
+  copy16<H * NOUT / 8>(W2c, a.W2c);
   if (tid == 0) mbar_init(mbar, 1);
   if (warp == 0) tmem_alloc(slot, kBwdCols);
   fence_async_smem();
@@ -1080,18 +1122,29 @@ __global__ void __launch_bounds__(32 * kReduceWarps)
 }
 
 // Flat FP32 parameters of one MLP -> padded BF16 weights and FP32 biases.
+// The canonical images follow in `canon`: W1 and W2 transposed (forward), then as
+// they are (backward).
 __global__ void k_pack(const float* p, int K1, int NOUT, int kin, int out, bf16* W1, float* b1,
-                       bf16* W2, float* b2) {
+                       bf16* W2, float* b2, bf16* canon) {
+  bf16* W2t = canon + K1 * H;
+  bf16* W1c = W2t + H * NOUT;
+  bf16* W2c = W1c + K1 * H;
   const int n = K1 * H + H + H * NOUT + NOUT;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     if (i < K1 * H) {
       const int r = i / H, c = i % H;
-      W1[i] = __float2bfloat16_rn(r < kin ? p[r * H + c] : 0.f);
+      const bf16 v = __float2bfloat16_rn(r < kin ? p[r * H + c] : 0.f);
+      W1[i] = v;
+      canon[canon_off(c, r, K1) / 2] = v;
+      W1c[canon_off(r, c, H) / 2] = v;
     } else if (i < K1 * H + H) {
       b1[i - K1 * H] = p[kin * H + (i - K1 * H)];
     } else if (i < K1 * H + H + H * NOUT) {
       const int k = i - K1 * H - H, r = k / NOUT, c = k % NOUT;
-      W2[k] = __float2bfloat16_rn(c < out ? p[kin * H + H + r * out + c] : 0.f);
+      const bf16 v = __float2bfloat16_rn(c < out ? p[kin * H + H + r * out + c] : 0.f);
+      W2[k] = v;
+      W2t[canon_off(c, r, H) / 2] = v;
+      W2c[canon_off(r, c, NOUT) / 2] = v;
     } else {
       const int c = i - K1 * H - H - H * NOUT;
       b2[c] = c < out ? p[kin * H + H + H * out + c] : 0.f;
@@ -1181,6 +1234,10 @@ struct Mlp {
   float* b1 = nullptr;
   bf16* W2 = nullptr;
   float* b2 = nullptr;
+  bf16* canon = nullptr;  // k_pack's images: W1t, W2t, W1c, W2c
+  const bf16* W2t() const { return canon + K1 * H; }
+  const bf16* W1c() const { return W2t() + H * NOUT; }
+  const bf16* W2c() const { return W1c() + K1 * H; }
 };
 
 }  // namespace gnn
@@ -1272,7 +1329,7 @@ int grid_for(plfbs_gnn* g, int M, int per_sm) {
 
 template <int MODE, int K1, int NOUT>
 int launch_fwd(plfbs_gnn* g, const Mlp& p, const Rows& x, float* z1, float* y) {
-  Fwd a{x, p.W1, p.b1, p.W2, p.b2, z1, y};
+  Fwd a{x, p.W1, p.b1, p.W2, p.b2, p.canon, p.W2t(), z1, y};
   if (g->use_tc) {
     // two blocks per SM: 2 x 98 KB of shared memory, 2 x 128 tensor-memory columns
     k_mlp_fwd_tc<MODE, K1, NOUT><<<grid_for(g, x.M, 2), kTcThreads, tc_smem<K1, NOUT>(),
@@ -1290,7 +1347,7 @@ template <int MODE, int K1, int NOUT>
 int launch_bwd(plfbs_gnn* g, const Mlp& p, const Rows& x, const float* dy, const float* dadd,
                const float* z1, float* dx0, float* dseg1, float* dseg2) {
   const int grid = grid_for(g, x.M, 1);
-  Bwd a{x, dy, dadd, z1, p.W1, p.W2, dx0, dseg1, dseg2, g->part};
+  Bwd a{x, dy, dadd, z1, p.W1, p.W2, p.W1c(), p.W2c(), dx0, dseg1, dseg2, g->part};
   if (g->use_tc)
     k_mlp_bwd_tc<MODE, K1, NOUT><<<grid, kTcThreads, bwd_tc_smem<K1, NOUT>(), g->stream>>>(
         a, g->tc_err);
@@ -1309,7 +1366,7 @@ Rows rows_enc(int M, const float* f) { return Rows{M, f, nullptr, nullptr, nullp
 int pack_all(plfbs_gnn* g) {
   for (const Mlp& p : g->mlps) {
     k_pack<<<64, 256, 0, g->stream>>>(g->params + p.off, p.K1, p.NOUT, p.kin, p.out, p.W1, p.b1,
-                                      p.W2, p.b2);
+                                      p.W2, p.b2, p.canon);
     GCK(cudaGetLastError());
   }
   return 0;
@@ -1493,7 +1550,8 @@ int plfbs_gnn_create(const plfbs_gnn_shape* shape, const int32_t* src, const int
     return fail(rc);
   for (Mlp& p : g->mlps) {
     if ((rc = galloc(g, &p.W1, (size_t)p.K1 * H)) || (rc = galloc(g, &p.b1, H)) ||
-        (rc = galloc(g, &p.W2, (size_t)H * p.NOUT)) || (rc = galloc(g, &p.b2, p.NOUT)))
+        (rc = galloc(g, &p.W2, (size_t)H * p.NOUT)) || (rc = galloc(g, &p.b2, p.NOUT)) ||
+        (rc = galloc(g, &p.canon, 2 * ((size_t)p.K1 * H + (size_t)H * p.NOUT))))
       return fail(rc);
   }
   // graph
