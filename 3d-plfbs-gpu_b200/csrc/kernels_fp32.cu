@@ -129,26 +129,39 @@ __device__ __forceinline__ void flux_face32(const KernelArgs& a, const int f, co
   stf(a.flux, f, face_flux32(a, n, f0.w, f2.w, sides, dt, si, sn, sc, g1, g2));
 }
 
-// Persistent over the faces, next face's ids prefetched (as k_flux); six blocks
-// per SM (85 registers) measured fastest.
+// Persistent over the faces, next face's ids prefetched, int counters and the
+// compact layout's block-uniform loop as in k_flux; six blocks per SM (85
+// registers) measured fastest.
 template <bool CR>
 __global__ void __launch_bounds__(kFluxBlock, 6) k_flux32(const KernelArgs a) {
   if (halted(a)) return;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= a.F) return;
-  int2 ids = __ldg(reinterpret_cast<const int2*>(a.face_ids) + f);
-  int rec = CR ? __ldg(a.face_rec + f) : 0;
-  for (;;) {
-    const long long fn = f + stride;
-    const int2 next =
-        fn < a.F ? __ldg(reinterpret_cast<const int2*>(a.face_ids) + fn) : make_int2(0, 0);
-    const int next_rec = (CR && fn < a.F) ? __ldg(a.face_rec + fn) : 0;
-    flux_face32<CR>(a, (int)f, ids, rec);
-    if (fn >= a.F) break;
-    f = fn;
-    ids = next;
-    rec = next_rec;
+  const int2* face_ids = reinterpret_cast<const int2*>(a.face_ids);
+  const int stride = gridDim.x * kFluxBlock;
+  int f = blockIdx.x * kFluxBlock + threadIdx.x;
+  if constexpr (CR) {
+    const int tiles = (a.F + kFluxBlock - 1) / kFluxBlock;
+    int2 ids = f < a.F ? __ldg(face_ids + f) : make_int2(0, 0);
+    int rec = f < a.F ? __ldg(a.face_rec + f) : 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+      const int fn = f + stride;
+      const int2 next = fn < a.F ? __ldg(face_ids + fn) : make_int2(0, 0);
+      const int next_rec = fn < a.F ? __ldg(a.face_rec + fn) : 0;
+      if (f < a.F) flux_face32<CR>(a, f, ids, rec);
+      f = fn;
+      ids = next;
+      rec = next_rec;
+    }
+  } else {
+    if (f >= a.F) return;
+    int2 ids = __ldg(face_ids + f);
+    for (;;) {
+      const int fn = f + stride;
+      const int2 next = fn < a.F ? __ldg(face_ids + fn) : make_int2(0, 0);
+      flux_face32<CR>(a, f, ids, 0);
+      if (fn >= a.F) break;
+      f = fn;
+      ids = next;
+    }
   }
 }
 
