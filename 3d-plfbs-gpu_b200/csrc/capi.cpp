@@ -1056,10 +1056,12 @@ int plfbs_run(plfbs_ctx* ctx, int64_t max_steps, plfbs_stats* stats, double* his
     const long long n = std::min<long long>(batch, max_steps - done);
     NvtxRange r("step batch");
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    if (marches(ctx->args))
+    if (marches(ctx->args)) {
       CK(plfbs::launch_march(ctx->args, ctx->cfg.precision, (int)n, ctx->stream));
-    else
+      ctx->grad_stale = ctx->flux_stale = true;  // also where the wait below runs out
+    } else {
       for (long long k = 0; k < n; k++) CK(cudaGraphLaunch(ctx->step_exec, ctx->stream));
+    }
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
     TRY(wait_steps(ctx, ctx->timeout_s));
     TRY(read_stats(ctx));
@@ -1082,7 +1084,6 @@ int plfbs_run(plfbs_ctx* ctx, int64_t max_steps, plfbs_stats* stats, double* his
     halt = ctx->stats_host->halt != 0;
     if (now - start == done && !halt)  // a batch that advanced nothing: never wait again
       return set_err(ctx, PLFBS_ERR_STATE, "the step graph made no progress");
-    if (now > start + done && marches(ctx->args)) ctx->grad_stale = ctx->flux_stale = true;
     done = now - start;
   }
   CK(cudaGetLastError());

@@ -114,3 +114,26 @@ def test_march_halts_at_the_step(plfbs_lib, precision):
         out.append(s.get_state())
         s.close()
     np.testing.assert_array_equal(out[0], out[1])
+
+
+def test_march_timed_out_leaves_no_old_gradients(plfbs_lib):
+    """A march whose wait ran out has still replaced the state that the
+    gradients and fluxes are read from."""
+    ma, c = _mesh("box", (12, 10, 9))
+    out = []
+    for timed_out in (True, False):
+        s = _solver(ma, c, capi.FP64, capi.FLAVOUR_GPU, 0)
+        s.set_state(_start(ma))
+        s.run_stages(4)
+        if timed_out:
+            s.set_timeout(1e-6)
+            with pytest.raises(capi.PlfbsError) as e:
+                s.run(300, history=False)
+            assert e.value.code == capi.ERR_TIMEOUT
+            assert s.wait(120.0)
+        else:
+            s.run(300, history=False)
+        out.append((s.gradients(), s.face_flux(), s.get_state()))
+        s.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
