@@ -203,7 +203,8 @@ int plfbs_polymesh_geometry(const plfbs_polymesh_view* mesh, double visc, double
 /* Replaces the setup half of Solver_gpu.cu:150-662: validates the views,
  * builds the least-squares weights (gradients.cpp:214-313), renumbers for
  * locality, uploads everything to `device` and captures one time step in a
- * CUDA graph. The mesh arrays are copied to the device first and checked
+ * CUDA graph; a mesh small enough for its tiles to sit in the SMs' shared
+ * memory gets them built instead and marches in one cooperative kernel. The mesh arrays are copied to the device first and checked
  * there (the same checks, first failing index and message as on the host
  * threads, which check them when `device` is absent); from page-locked host
  * memory the copies set the pace. The initial state is all zeros until
@@ -286,7 +287,8 @@ int plfbs_get_body_force(plfbs_ctx* ctx, double frontal_area, double* cd, double
 
 /* Introspection for parity tests (caller numbering). plfbs_run_stages advances
  * by RK stages (4 per time step; the IBM update runs before each step's first
- * stage) with individual kernel launches instead of the step graph. The
+ * stage) with individual kernel launches instead of the step graph or the
+ * marching kernel, and gives the same bits. The
  * getters return the last stage's interior-cell gradients [12C] (rho, u, v, w,
  * each x, y, z), face fluxes [4F] (x, y, z momentum, mass) and residuals [4C]
  * (u, v, w, rho); residuals are only recorded after plfbs_set_debug(ctx, 1). */
