@@ -184,8 +184,8 @@ __device__ __forceinline__ unsigned pair_side(const double n[3], double d1) {
 // every warp.
 //
 // The kernels that call this are bound by the FP64 pipe and the latency of
-// their gathers, so the sum is arranged for the fewest FP64 instructions (about
-// 295 per face of an axis-aligned mesh, 375 with a separate evaluation per
+// their gathers, so the sum is arranged for the fewest FP64 instructions
+// (298 per face on tetrahedra, 372-375 with a separate evaluation per
 // node; k_flux on the 256x128x128 channel 487 -> 447 us, on 1.57 M tetrahedra
 // 155 -> 148 us):
 //  - A side's field value at a diagonal node is (s -+ dt gz) -+ dt (gx +- gy):

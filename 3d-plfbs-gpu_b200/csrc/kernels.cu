@@ -1,7 +1,9 @@
 // sm_100a kernels of the LBFS explicit time step (FP64 path).
 //
 // One RK stage is three kernels, and a time step is the IBM kernel plus four
-// stages, all captured in one CUDA graph by capi.cpp:
+// stages, all captured in one CUDA graph by capi.cpp (a mesh small enough
+// marches in one cooperative kernel instead, march.cu, and uses these stage by
+// stage only):
 //
 //   gradient  (thread per cell)  ghost states inline + least-squares gradient
 //                                 [get_interior_gradients, update_unstructured_bcs]
