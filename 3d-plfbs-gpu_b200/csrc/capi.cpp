@@ -177,10 +177,39 @@ void give_pinned_staging(void* p, size_t n) {
 
 
 
-// One time step: IBM, then 4 x (gradient, flux, update) (Solver_gpu.cu:667-833).
-// Whether a run takes the march kernel instead of the step graph.
+// Whether a run can take the march kernel instead of the step graph.
 bool marches(const KernelArgs& a) { return a.tiles.n > 0 && !a.flux_maps && !a.res_debug; }
 
+// The SMs that the runs in flight on each device want at once: a march's tiles,
+// or the whole device for a context without. A march holds its SMs for a batch
+// of steps, so marches that fit beside each other run at their own pace (eight
+// of 12 tiles: 3.7 us per step and solve, 8.2 with step graphs), while full
+// ones would take turns (four threads, 32^3 cavity: 40 us per step and solve;
+// 64x32x32 channel 67 FP64, 48 FP32) where the kernels of step graphs fill each
+// other's gaps (27, 52 and 31). So a batch marches if the tiles of all runs in
+// flight fit; the results are the same bits either way.
+constexpr int kWholeDevice = 1 << 12;
+// Steps of a march until the next look at what else is in flight, 15 to 35 ms
+// (its wait and launch cost about 40 us); with a limit on the host's waits a
+// batch is always the full one.
+constexpr int kMarchSteps = 512;
+std::atomic<int> g_sms_wanted[plfbs::kMaxDevices];
+
+struct InFlight {
+  std::atomic<int>& wanted;
+  const int n;
+  explicit InFlight(const plfbs_ctx* ctx)
+      : wanted(g_sms_wanted[ctx->device >= 0 && ctx->device < plfbs::kMaxDevices ? ctx->device : 0]),
+        n(marches(ctx->args) ? ctx->args.tiles.n : kWholeDevice) {
+    wanted += n;
+  }
+  ~InFlight() { wanted -= n; }
+  InFlight(const InFlight&) = delete;
+  InFlight& operator=(const InFlight&) = delete;
+  bool march_fits(int sms) const { const int w = wanted; return w == n || w <= sms; }
+};
+
+// One time step: IBM, then 4 x (gradient, flux, update) (Solver_gpu.cu:667-833).
 void enqueue_step(const KernelArgs& a, int prec, cudaStream_t s) {
   plfbs::launch_ibm(a, prec, s);
   for (int rk = 0; rk < 4; rk++) {
@@ -190,12 +219,7 @@ void enqueue_step(const KernelArgs& a, int prec, cudaStream_t s) {
   }
 }
 
-int capture_step(plfbs_ctx* ctx) {
-  if (ctx->step_exec) {
-    cudaGraphExecDestroy(ctx->step_exec);
-    ctx->step_exec = nullptr;
-  }
-  if (marches(ctx->args)) return PLFBS_OK;  // no graph
+int build_graph(plfbs_ctx* ctx) {
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   enqueue_step(ctx->args, ctx->cfg.precision, ctx->stream);
@@ -205,6 +229,15 @@ int capture_step(plfbs_ctx* ctx) {
   if (e != cudaSuccess)
     return set_err(ctx, PLFBS_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
   return PLFBS_OK;
+}
+
+int capture_step(plfbs_ctx* ctx) {
+  if (ctx->step_exec) {
+    cudaGraphExecDestroy(ctx->step_exec);
+    ctx->step_exec = nullptr;
+  }
+  if (marches(ctx->args)) return PLFBS_OK;  // a graph once a batch needs it
+  return build_graph(ctx);
 }
 
 int reset_force(plfbs_ctx* ctx) {
@@ -1052,15 +1085,20 @@ int plfbs_run(plfbs_ctx* ctx, int64_t max_steps, plfbs_stats* stats, double* his
   float ms_total = 0.f;
   const long long batch = plfbs::kHistoryCap / 2;
   bool halt = ctx->stats_host->halt != 0;
+  const InFlight in_flight(ctx);
   while (done < max_steps && !halt) {
-    const long long n = std::min<long long>(batch, max_steps - done);
     NvtxRange r("step batch");
+    const bool march = marches(ctx->args) && in_flight.march_fits(ctx->sms);
+    const long long n = std::min<long long>(
+        march && ctx->timeout_s == 0 ? kMarchSteps : batch, max_steps - done);
+    if (!march && !ctx->step_exec) TRY(build_graph(ctx));
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    if (marches(ctx->args)) {
+    if (march) {
       CK(plfbs::launch_march(ctx->args, ctx->cfg.precision, (int)n, ctx->stream));
       ctx->grad_stale = ctx->flux_stale = true;  // also where the wait below runs out
     } else {
       for (long long k = 0; k < n; k++) CK(cudaGraphLaunch(ctx->step_exec, ctx->stream));
+      ctx->grad_stale = ctx->flux_stale = false;
     }
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
     TRY(wait_steps(ctx, ctx->timeout_s));

@@ -21,6 +21,7 @@ struct plfbs_ctx {
   int N = 0;
   cudaStream_t stream = nullptr;
   cudaGraphExec_t step_exec = nullptr;
+  int sms = 0;  // of the device (set for meshes that may march)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   plfbs::KernelArgs args{};
   std::vector<void*> allocs;

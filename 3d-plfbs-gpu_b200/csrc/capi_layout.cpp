@@ -386,6 +386,7 @@ int build_tiles(plfbs_ctx* ctx) {
   CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
   CK(cudaDeviceGetAttribute(&most_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
   most_smem -= 4096;  // the kernel's own arrays
+  ctx->sms = sms;
   const int tiles = std::min(sms, plfbs::march_max_tiles());
   plfbs::TileArgs t{};
   t.T = ((a.C + tiles - 1) / tiles + 31) / 32 * 32;

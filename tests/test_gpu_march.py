@@ -5,6 +5,8 @@ fluxes agree bit for bit, over cell counts at the edges of the tiles, both
 precisions and flavours, with and without the compact layout, and where the
 context halts in the middle of a march."""
 
+import threading
+
 import numpy as np
 import pytest
 
@@ -137,3 +139,28 @@ def test_march_timed_out_leaves_no_old_gradients(plfbs_lib):
         s.close()
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [(11, 3, 1), (37, 16, 8)])  # 2 tiles; one per SM
+def test_march_beside_other_runs(plfbs_lib, n):
+    """Runs on several threads take the march or the step graph batch by batch,
+    by what else is in flight: the same bits as the run alone."""
+    ma, c = _mesh("box", n)
+    out = [None] * 4
+
+    def solve(k, calls):
+        s = _solver(ma, c, capi.FP64, capi.FLAVOUR_GPU, 0)
+        s.set_state(_start(ma))
+        h = [s.run(30)[1] for _ in range(calls)]
+        out[k] = (np.concatenate(h), s.gradients(), s.face_flux(), s.get_state())
+        s.close()
+
+    solve(0, 10)
+    threads = [threading.Thread(target=solve, args=(k, 10)) for k in (1, 2, 3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in (1, 2, 3):
+        for a, b in zip(out[0], out[k]):
+            np.testing.assert_array_equal(a, b)
