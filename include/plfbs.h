@@ -203,9 +203,10 @@ int plfbs_polymesh_geometry(const plfbs_polymesh_view* mesh, double visc, double
 /* Replaces the setup half of Solver_gpu.cu:150-662: validates the views,
  * builds the least-squares weights (gradients.cpp:214-313), renumbers for
  * locality, uploads everything to `device` and captures one time step in a
- * CUDA graph; a mesh small enough for its tiles to sit in the SMs' shared
- * memory gets them built instead and marches in one cooperative kernel (while runs
- * of other contexts need its SMs too, in step graphs, with the same results). The mesh arrays are copied to the device first and checked
+ * CUDA graph. A mesh small enough for its tiles to sit in the SMs' shared
+ * memory gets them built instead and marches in one cooperative kernel; while
+ * runs of other contexts want its SMs too it takes step graphs, with the same
+ * results. The mesh arrays are copied to the device first and checked
  * there (the same checks, first failing index and message as on the host
  * threads, which check them when `device` is absent); from page-locked host
  * memory the copies set the pace. The initial state is all zeros until
