@@ -444,6 +444,7 @@ int build_tiles(plfbs_ctx* ctx) {
   plfbs::launch_tile_build(a, ctx->curve, pos, side, t, got[0], got[1], ctx->stream);
   CK(cudaGetLastError());
   a.tiles = t;
+  CK(plfbs::prepare_march(a, prec, most_smem));
   a.red_order = ctx->curve;
   a.red_warps = t.T / 32;
   return PLFBS_OK;

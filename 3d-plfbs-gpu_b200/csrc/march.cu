@@ -701,13 +701,28 @@ int march_smem(const KernelArgs& a, int precision, int most, TileArgs& t) {
   return n <= (size_t)most ? (int)n : 0;
 }
 
+// The attribute belongs to the kernel on the device, not to a context: threads
+// launch the same instance with tiles of different sizes, so every context sets
+// the same value, the device's limit.
+cudaError_t prepare_march(const KernelArgs& a, int precision, int most) {
+  cudaError_t e = cudaSuccess;
+  KernelArgs args = a;
+  for (int k = 0; k < 2 && e == cudaSuccess; k++) {
+    e = with_form(args, precision, [&](auto f) {
+      using Fm = decltype(f);
+      return cudaFuncSetAttribute(k_march<Fm, march_threads<Fm>()>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    });
+    args.compact = 0;  // plfbs_set_layout_compression
+  }
+  return e;
+}
+
 cudaError_t launch_march(const KernelArgs& a, int precision, int nsteps, cudaStream_t s) {
   return with_form(a, precision, [&](auto f) {
     using Fm = decltype(f);
     constexpr int NT = march_threads<Fm>();
-    cudaError_t e = cudaFuncSetAttribute(k_march<Fm, NT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, a.tiles.smem);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a.grid_bar, 0, sizeof(unsigned), s);
+    const cudaError_t e = cudaMemsetAsync(a.grid_bar, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
     KernelArgs args = a;
     int n = nsteps;

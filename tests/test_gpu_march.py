@@ -164,3 +164,35 @@ def test_march_beside_other_runs(plfbs_lib, n):
     for k in (1, 2, 3):
         for a, b in zip(out[0], out[k]):
             np.testing.assert_array_equal(a, b)
+
+
+def test_march_tiles_of_different_sizes_on_three_threads(plfbs_lib):
+    """The largest dynamic shared memory of a kernel is one value per device:
+    meshes whose tiles take different amounts, one of them more than the 48 KB a
+    kernel has without asking, and fit on the SMs together (144, 2 and 2 of 148)
+    march on three threads in many short runs."""
+    errs, out = [], {}
+
+    def solve(n, runs, key):
+        try:
+            ma, c = _mesh("box", n)
+            s = _solver(ma, c, capi.FP64, capi.FLAVOUR_GPU, 0)
+            s.set_state(_start(ma))
+            for _ in range(runs):
+                s.run(1, history=False)
+            out[key] = s.get_state()
+            s.close()
+        except capi.PlfbsError as e:
+            errs.append((n, repr(e)))
+
+    meshes = [(24, 24, 24), (11, 3, 1), (1, 33, 1)]
+    for n in meshes:
+        solve(n, 4000, n)
+    threads = [threading.Thread(target=solve, args=(n, 4000, n + (0,))) for n in meshes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errs, errs
+    for n in meshes:
+        np.testing.assert_array_equal(out[n], out[n + (0,)])
