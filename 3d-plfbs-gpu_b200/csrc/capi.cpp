@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "capi_internal.hpp"
+#include "eq_constants.hpp"
 
 using plfbs::DevStats;
 using plfbs::KernelArgs;
@@ -596,9 +597,13 @@ int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh, const plf
   a.nblk_update = (L.C + plfbs::kBlock - 1) / plfbs::kBlock;
   a.dt = cfg->time_marching_step;
   a.pg = 1.0 / cfg->gamma;
-  a.eq_k0 = cfg->gamma / 1.5;
-  a.eq_k1 = 2.0 * cfg->gamma;
-  a.eq_cd = 1.5 / 72.0 / cfg->gamma;
+  {
+    const auto k = plfbs::eq_constants64(cfg->gamma);
+    a.eq_k0 = k.k0;
+    a.eq_k1 = k.k1;
+    a.eq_cd = k.cd;
+    a.eq_cd3 = k.cd / 3;
+  }
   a.visc3 = cfg->visc * 3;
   // body force: +pressure_gradient on the GPU path (Solver_gpu.cu:700), the
   // CPU Solver's force = -pressure_gradient (Solver.cpp:213)
@@ -611,11 +616,11 @@ int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh, const plf
   a.rho0 = cfg->ref_rho;
   a.uref = cfg->max_velocity;
   {
-    const double c = 1.5 * a.uref * a.uref * a.pg;
-    a.eq32_k0 = (float)(1.0 / c);
-    a.eq32_k1 = (float)(2.0 * cfg->gamma / a.uref);
-    a.eq32_cd = (float)(c / 72.0);
-    a.eq32_pgcd = (float)(c / 72.0 * a.pg);
+    const auto k = plfbs::eq_constants32(cfg->gamma, a.uref);
+    a.eq32_k0 = k.k0;
+    a.eq32_k1 = k.k1;
+    a.eq32_cd = k.cd;
+    a.eq32_pgcd = (float)(k.cd * a.pg);
   }
   a.rho0f = (float)cfg->ref_rho;
   a.inv_uref_f = (float)(1.0 / cfg->max_velocity);

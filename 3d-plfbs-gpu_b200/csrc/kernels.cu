@@ -137,12 +137,11 @@ __device__ __forceinline__ void flux_face(const KernelArgs& a, const int f, cons
     load_grad(a.grad, nb, g2);
     if (CR && (sides >> kKindShift)) {
       const double2 w = __ldg(reinterpret_cast<const double2*>(a.frec_relax) + r);
-      const double cA = __dmul_rn(f0.w, a.eq_cd);
       const unsigned kind = sides >> kKindShift;
       const d4 x =
-          kind == 1 ? axis_flux<FL, 0>(a, dt, t1[0], t2[0], f0.x, cA, w.x, w.y, qo, qn, g1, g2)
-          : kind == 2 ? axis_flux<FL, 1>(a, dt, t1[1], t2[1], f0.y, cA, w.x, w.y, qo, qn, g1, g2)
-                      : axis_flux<FL, 2>(a, dt, t1[2], t2[2], f0.z, cA, w.x, w.y, qo, qn, g1, g2);
+          kind == 1 ? axis_flux<FL, 0>(a, dt, t1[0], t2[0], f0.x, f0.w, w.x, w.y, qo, qn, g1, g2)
+          : kind == 2 ? axis_flux<FL, 1>(a, dt, t1[1], t2[1], f0.y, f0.w, w.x, w.y, qo, qn, g1, g2)
+                      : axis_flux<FL, 2>(a, dt, t1[2], t2[2], f0.z, f0.w, w.x, w.y, qo, qn, g1, g2);
       st4(a.flux, f, x);
       return;
     }

@@ -100,17 +100,18 @@ struct Form64 {
     double R, m[3], P[6];
     face_moments<FL>(a.eq_k0, a.eq_k1, f1.x, sides, si, sn, sc, g1, g2, R, m, P);
     const V f0 = ST ? row(tab, r, 0) : rec[0];
-    const double n[3] = {f0.x, f0.y, f0.z}, cA = __dmul_rn(f0.w, a.eq_cd);
+    const double n[3] = {f0.x, f0.y, f0.z};
     double omA, tA;  // as face_flux forms them
     if (ST) {
       const double2 w = *reinterpret_cast<const double2*>(tab + r * kRecRow + 12);
       omA = w.x;
       tA = w.y;
     } else {
+      const double cA = __dmul_rn(f0.w, a.eq_cd);
       omA = __dmul_rn(__dadd_rn(1.0, -f2.w), cA);
       tA = __dmul_rn(f2.w, cA);
     }
-    return flux_of_moments(a.pg, R, m, P, n, cA, omA, tA);
+    return flux_of_moments(a, R, m, P, n, f0.w, omA, tA);
   }
   template <int RK>
   static __device__ __forceinline__ void rk(const KernelArgs& a, const V& t0, const V& t1,

@@ -331,9 +331,9 @@ struct KernelArgs {
   // scalars
   double dt;            // RK time step
   double pg;            // 1 / gamma
-  // equilibrium constants of the flux (flux_core.cuh): 2 gamma / 3, 2 gamma
-  // and the moments' unit, 1 / (48 gamma)
-  double eq_k0, eq_k1, eq_cd;
+  // equilibrium constants of the flux (eq_constants.hpp): 2 gamma / 3, 2 gamma
+  // the moments' unit cd, 1 / (48 gamma), and cd / 3
+  double eq_k0, eq_k1, eq_cd, eq_cd3;
   double visc3;         // 3 nu (relaxation factor is 3 nu / (dt_s gamma))
   double pressure_gradient;
   double tolerance;
