@@ -179,7 +179,10 @@ void give_pinned_staging(void* p, size_t n) {
 
 
 // Whether a run can take the march kernel instead of the step graph.
-bool marches(const KernelArgs& a) { return a.tiles.n > 0 && !a.flux_maps && !a.res_debug; }
+bool marches(const KernelArgs& a) {
+  return a.tiles.n > 0 && (a.tiles.own || (a.compact && a.face_rec && a.wtab)) && !a.flux_maps &&
+         !a.res_debug;
+}
 
 // The SMs that the runs in flight on each device want at once: a march's tiles,
 // or the whole device for a context without. A march holds its SMs for a batch

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "capi_internal.hpp"
+#include "march_rules.hpp"
 
 using plfbs::KernelArgs;
 using plfbs::Layout;
@@ -369,15 +370,8 @@ int device_cell_order(plfbs_ctx* ctx, const plfbs_mesh_view& m, std::vector<int3
 }
 
 // One tile per SM, so the mesh must fit them all at once: a tile's rows in a
-// block's shared memory and its indices in the tables' widths (up to about
-// 68,000 FP64 or 142,000 FP32 hexahedra on 148 SMs). Within that the march wins
-// where the face records are few and shared (FP64 hexahedra: 512 cells 25 us
-// per step against 57 with the kernels one by one, 27,648 cells 41 : 76, 64,000
-// cells 64 : 86; FP32 128,000 cells 70 : 85). With records of their own its
-// blocks wait for them at every face, so it takes the mesh up to
-// kMarchFaces64 / kMarchFaces32 faces per SM (FP64: 131,000 faces 70 us : 78, but
-// 170,000 90 : 82; FP32: 170,000 55 : 64, 320,000 153 : 78).
-constexpr int kMarchFaces64 = 900, kMarchFaces32 = 1600;
+// block's shared memory and its indices in the tables' widths; and the march
+// must be the faster one (march_rules.hpp) in the form the mesh is in.
 int build_tiles(plfbs_ctx* ctx) {
   KernelArgs& a = ctx->args;
   const int prec = ctx->cfg.precision;
@@ -392,10 +386,8 @@ int build_tiles(plfbs_ctx* ctx) {
   t.T = ((a.C + tiles - 1) / tiles + 31) / 32 * 32;
   if (!coop || t.T > plfbs::march_max_own() || a.F >= (1 << 28) || !ctx->curve)
     return PLFBS_OK;
-  const bool shared = a.face_rec && a.wtab;  // the compact layout
-  if (!shared &&
-      a.F > tiles * (prec == PLFBS_FP32_DEVIATION ? kMarchFaces32 : kMarchFaces64))
-    return PLFBS_OK;
+  const bool fp32 = prec == PLFBS_FP32_DEVIATION, compact = a.face_rec && a.wtab;
+  if (!plfbs::march_may_win(compact, fp32, tiles, a.F)) return PLFBS_OK;
   t.n = (a.C + t.T - 1) / t.T;
   ScratchList S(ctx);
   int32_t *most = nullptr, *pos = nullptr;
@@ -415,6 +407,9 @@ int build_tiles(plfbs_ctx* ctx) {
   t.smem = plfbs::march_smem(a, prec, most_smem, t);
   if (t.T + got[1] > plfbs::kTileMaxCells || got[0] > plfbs::kTileMaxFaces || t.smem == 0)
     return PLFBS_OK;
+  t.own = plfbs::march_may_win(false, fp32, tiles, a.F) &&
+          plfbs::march_wins(false, fp32, t.n, t.SF, a.F);
+  if (!t.own && !(compact && plfbs::march_wins(true, fp32, t.n, t.SF, a.F))) return PLFBS_OK;
   const size_t cells = (size_t)t.n * t.SC, faces = (size_t)t.n * t.SF;
   void* p = nullptr;
   TRY(pool_alloc(ctx, &p, 4 * cells));
@@ -437,7 +432,7 @@ int build_tiles(plfbs_ctx* ctx) {
   t.slot = static_cast<uint16_t*>(p);
   TRY(pool_alloc(ctx, &p, sizeof(int2) * (size_t)t.n));
   t.count = static_cast<int2*>(p);
-  TRY(pool_alloc(ctx, &p, (prec == PLFBS_FP32_DEVIATION ? 16 : 32) * ((size_t)a.C + a.B)));
+  TRY(pool_alloc(ctx, &p, (fp32 ? 16 : 32) * ((size_t)a.C + a.B)));
   a.state2 = p;
   TRY(pool_alloc(ctx, &p, sizeof(unsigned)));
   a.grid_bar = static_cast<unsigned*>(p);

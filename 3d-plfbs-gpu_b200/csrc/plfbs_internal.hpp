@@ -306,6 +306,7 @@ struct TileArgs {
   int smem;  // dynamic shared memory of a block
   int tables;  // 1: the compact tables are copied there
   int place;   // the tile's tables there: 1 slot, 2 ij and rec / fid, 4 cell, nbr, wset
+  int own;     // 1: the march is also the faster one with a record per face (march_rules.hpp)
   int32_t* cell;
   int32_t* nbr;
   int32_t* wset;

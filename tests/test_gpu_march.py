@@ -196,3 +196,82 @@ def test_march_tiles_of_different_sizes_on_three_threads(plfbs_lib):
     assert not errs, errs
     for n in meshes:
         np.testing.assert_array_equal(out[n], out[n + (0,)])
+
+
+def _same_run(ma, c, precision, flavour, want_compact, mode=None, compress=None, ibm=None,
+              exact=True):
+    """As _same, on given mesh arrays (want_compact: whether the face records and
+    the weight sets of the layout repeat) and with an immersed body."""
+    out = []
+    for march in (True, False):
+        rt, vt, val = cases.bc_arrays(ma, c)
+        cfg = dict(visc=c.visc, dt=c.dt, max_velocity=c.mach, channel_height=c.Y,
+                   lengths=(c.X, c.Y, c.Z), flavour=flavour, precision=precision,
+                   pressure_gradient=1e-5, domain_dt=0.5,
+                   gradient_mode=mode or (capi.GRAD_LS | capi.GRAD_EXACT_INVERSE))
+        s = capi.Solver(ma, rt, vt, val, cfg, ibm=ibm)
+        got = s.layout()["compact"]
+        assert (got[0] > 0, got[1] > 0) == want_compact, got
+        if all(want_compact):
+            assert max(got) > 32  # not the form with the tables in shared memory
+        if compress is not None:
+            s.set_layout_compression(compress)
+        s.set_state(_start(ma))
+        if march:
+            s.run(STEPS)
+        else:
+            s.run_stages(4 * STEPS)
+        out.append((s.gradients(), s.face_flux(), s.get_state()) + (s.nodes() if ibm else ()))
+        s.close()
+    assert np.isfinite(out[0][2]).all()
+    for a, b in zip(*out):
+        if exact:
+            np.testing.assert_array_equal(a, b)
+        else:  # atomic sums of the body's forces in any order
+            tol = 1e-12 if precision == capi.FP64 else 2e-5
+            np.testing.assert_allclose(a, b, rtol=0, atol=tol * max(1.0, np.abs(b).max()))
+
+
+FORMS = [(capi.FP64, capi.FLAVOUR_GPU), (capi.FP64, capi.FLAVOUR_CPU_SOLVER),
+         (capi.FP32_DEVIATION, capi.FLAVOUR_GPU)]
+
+
+# the compact layout with more records than the shared-memory tables take (along
+# each axis), and with only the face records or only the weight sets repeating
+@pytest.mark.parametrize("form", ["x", "y", "z", "faces", "weights"])
+@pytest.mark.parametrize("precision,flavour", FORMS)
+def test_march_is_the_stages_compact_forms(plfbs_lib, form, precision, flavour):
+    n, mode = (21, 22, 23), None
+    grid = [np.arange(k + 1.0) for k in n]
+    if form in "xyz":
+        k = "xyz".index(form)
+        grid[k] = np.concatenate([[0.0], np.cumsum(1 + np.arange(n[k]) / 64)])  # exact sums
+    sides = ["inlet", "outlet", "side", "side", "side", "side"]
+    c = _mesh("box", (2, 2, 2))[1]
+    ma = cases.mesh_arrays(cases.hex_box(*grid, patch_types=sides), c.visc, c.gamma, c.fneq_min)
+    rng = np.random.default_rng(7)
+    want = (True, True)
+    if form == "weights":  # every face a streaming time of its own
+        ma.streaming_dt = np.asarray(ma.streaming_dt) * rng.uniform(0.9, 1.0, len(ma.streaming_dt))
+        want = (False, True)
+    if form == "faces":  # every cell a hybrid weight of its own
+        ma.cell_volume = np.array(ma.cell_volume) * rng.uniform(0.9, 0.99, len(ma.cell_volume))
+        mode, want = capi.GRAD_HYBRID | capi.GRAD_EXACT_INVERSE, (True, False)
+    _same_run(ma, c, precision, flavour, want, mode)
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.FP32_DEVIATION])
+@pytest.mark.parametrize("nodes", [1, 60])
+def test_march_is_the_stages_with_a_body(plfbs_lib, precision, nodes):
+    """The body's nodes inside a march: one node, whose eight cells get a force
+    each, to the bit, and a sphere to the rounding of its atomic sums."""
+    c = _mesh("box", (2, 2, 2))[1]
+    n = (24, 16, 16)
+    c.X, c.Y, c.Z = n
+    grid = [np.arange(k + 1.0) for k in n]
+    grid[2] = np.concatenate([[0.0], np.cumsum(1 + np.arange(n[2]) / 1024)])
+    ma = cases.mesh_arrays(cases.hex_box(*grid, patch_types=["inlet", "outlet"] + ["side"] * 4),
+                           c.visc, c.gamma, c.fneq_min)
+    x = cases.fibonacci_sphere(nodes, 2.0, (8.0, 8.0, 8.0))
+    ibm = dict(node_ref=x, stiffness=0.5, radius=2.0, depth=4.0, object_nodes=max(nodes, 2))
+    _same_run(ma, c, precision, capi.FLAVOUR_GPU, (True, True), ibm=ibm, exact=nodes == 1)
