@@ -649,7 +649,8 @@ int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh, const plf
   {
     NvtxRange r("device layout");
     if ((rc = build_device_layout(ctx, *mesh))) return fail(rc);
-    free_stage(ctx);  // stream-ordered: after the layout kernels that read it
+    // stream-ordered: after the layout kernels that read it
+    if (L.C > plfbs::march_max_tiles() * plfbs::march_max_own()) free_stage(ctx);
   }
   {
     NvtxRange r("compact layout");
@@ -658,6 +659,7 @@ int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh, const plf
   {
     NvtxRange r("tiles");
     if ((rc = build_tiles(ctx))) return fail(rc);
+    free_stage(ctx);
   }
   if (ctx->pre.bc[0]) {  // copied while the mesh copies ran
     a.bc0 = ctx->pre.bc[0];

@@ -39,7 +39,6 @@ struct plfbs_ctx {
   int compact_faces = 0;          // unique face records in the compact layout (0: none)
   int compact_cells = 0;          // unique cell weight sets in the compact layout (0: none)
   bool flux_maps_ok = false;
-  int32_t* curve = nullptr;       // device [C]: the cells along a space-filling curve
   // gradients and fluxes on the device are older than the last step (the
   // march kernel does not write them); recomputed when asked for
   bool grad_stale = false, flux_stale = false;

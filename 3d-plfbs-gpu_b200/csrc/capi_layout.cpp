@@ -190,26 +190,6 @@ int build_device_layout(plfbs_ctx* ctx, const plfbs_mesh_view& m) {
   ctx->perm = static_cast<int32_t*>(p);
   plfbs::launch_perm(d.cell_new, d.bc_new, L.C, L.B, ctx->perm, ctx->stream);
   CK(cudaGetLastError());
-  // the cells along a space-filling curve, for the tiles of a mesh small
-  // enough to have them (build_tiles)
-  if (L.C <= plfbs::march_max_tiles() * plfbs::march_max_own()) {
-    const plfbs::CurveSizes z = plfbs::curve_sizes(L.C);
-    plfbs::CurveScratch c{};
-    TRY(S.alloc(&c.part, 8 * z.part, false));
-    for (int k = 0; k < 2; k++) {
-      TRY(S.alloc(&c.key[k], 4 * C, false));
-      TRY(S.alloc(&c.val[k], 4 * C, false));
-    }
-    TRY(S.alloc(&c.count, 4 * z.count, false));
-    TRY(S.alloc(&c.off, 4 * z.count, false));
-    TRY(S.alloc(&c.wsum, 4 * z.windows, false));
-    TRY(S.alloc(&c.wbase, 4 * (z.windows + 1), false));
-    TRY(S.alloc(&c.info, 16, true));
-    TRY(pool_alloc(ctx, &p, 4 * C));
-    ctx->curve = static_cast<int32_t*>(p);
-    plfbs::launch_cell_curve(d, c, ctx->curve, ctx->stream);
-    CK(cudaGetLastError());
-  }
   plfbs::LayoutScratch s{};
   TRY(S.alloc(&s.own_cnt, 4 * C, true));
   TRY(S.alloc(&s.own_off, 4 * C, false));
@@ -384,19 +364,38 @@ int build_tiles(plfbs_ctx* ctx) {
   const int tiles = std::min(sms, plfbs::march_max_tiles());
   plfbs::TileArgs t{};
   t.T = ((a.C + tiles - 1) / tiles + 31) / 32 * 32;
-  if (!coop || t.T > plfbs::march_max_own() || a.F >= (1 << 28) || !ctx->curve)
+  if (!coop || t.T > plfbs::march_max_own() || a.F >= (1 << 28) || !ctx->stage.ok)
     return PLFBS_OK;
   const bool fp32 = prec == PLFBS_FP32_DEVIATION, compact = a.face_rec && a.wtab;
   if (!plfbs::march_may_win(compact, fp32, tiles, a.F)) return PLFBS_OK;
   t.n = (a.C + t.T - 1) / t.T;
   ScratchList S(ctx);
-  int32_t *most = nullptr, *pos = nullptr;
+  int32_t *curve = nullptr, *most = nullptr, *pos = nullptr;
   uint16_t* side = nullptr;
+  {  // the cells along a space-filling curve
+    const size_t C = (size_t)a.C;
+    const plfbs::CurveSizes z = plfbs::curve_sizes(a.C);
+    plfbs::CurveScratch c{};
+    TRY(S.alloc(&c.part, 8 * z.part, false));
+    for (int k = 0; k < 2; k++) {
+      TRY(S.alloc(&c.key[k], 4 * C, false));
+      TRY(S.alloc(&c.val[k], 4 * C, false));
+    }
+    TRY(S.alloc(&c.count, 4 * z.count, false));
+    TRY(S.alloc(&c.off, 4 * z.count, false));
+    TRY(S.alloc(&c.wsum, 4 * z.windows, false));
+    TRY(S.alloc(&c.wbase, 4 * (z.windows + 1), false));
+    TRY(S.alloc(&c.info, 16, true));
+    TRY(S.alloc(&curve, 4 * C, false));
+    plfbs::launch_cell_curve(a.C, ctx->stage.ccen, ctx->stage.vol, a.ibm_map, c, curve,
+                             ctx->stream);
+    CK(cudaGetLastError());
+  }
   TRY(S.alloc(&most, 8, true));
   TRY(S.alloc(&side, 2 * (size_t)a.F, false));
   TRY(S.alloc(&pos, 4 * (size_t)a.C, false));
-  plfbs::launch_tile_order(a.C, t.T, ctx->curve, pos, ctx->stream);
-  plfbs::launch_tile_count(a, ctx->curve, pos, t.T, most, ctx->stream);
+  plfbs::launch_tile_order(a.C, t.T, curve, pos, ctx->stream);
+  plfbs::launch_tile_count(a, curve, pos, t.T, most, ctx->stream);
   plfbs::launch_face_sides(a, prec, side, ctx->stream);
   CK(cudaGetLastError());
   int32_t got[2];
@@ -436,11 +435,13 @@ int build_tiles(plfbs_ctx* ctx) {
   a.state2 = p;
   TRY(pool_alloc(ctx, &p, sizeof(unsigned)));
   a.grid_bar = static_cast<unsigned*>(p);
-  plfbs::launch_tile_build(a, ctx->curve, pos, side, t, got[0], got[1], ctx->stream);
+  plfbs::launch_tile_build(a, curve, pos, side, t, got[0], got[1], ctx->stream);
   CK(cudaGetLastError());
   a.tiles = t;
   CK(plfbs::prepare_march(a, prec, most_smem));
-  a.red_order = ctx->curve;
+  TRY(pool_alloc(ctx, &p, 4 * (size_t)a.C));
+  CK(cudaMemcpyAsync(p, curve, 4 * (size_t)a.C, cudaMemcpyDeviceToDevice, ctx->stream));
+  a.red_order = static_cast<const int32_t*>(p);
   a.red_warps = t.T / 32;
   return PLFBS_OK;
 }

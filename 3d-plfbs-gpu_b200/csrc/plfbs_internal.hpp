@@ -438,8 +438,8 @@ struct CurveSizes {
   size_t part, count, windows;
 };
 CurveSizes curve_sizes(int C);
-void launch_cell_curve(const DevMesh& m, const CurveScratch& s, int32_t* order,
-                       cudaStream_t stream);
+void launch_cell_curve(int C, const double* ccen, const double* vol, const int32_t* cell_new,
+                       const CurveScratch& s, int32_t* order, cudaStream_t stream);
 // Cut into tiles of T cells, each sorted by device index, and the inverse.
 void launch_tile_order(int C, int T, int32_t* order, int32_t* pos, cudaStream_t stream);
 // The tile tables: branch bits of all faces, the largest tile's faces and cut

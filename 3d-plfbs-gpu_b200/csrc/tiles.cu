@@ -27,16 +27,17 @@ constexpr int kSortItems = 4096;  // items per block of the radix sort: 8 warps 
 
 // Per-block bounds of the centroids and sums of the volumes, in a fixed
 // partition and order, so that every context of a mesh gets the same tiles.
-__global__ void __launch_bounds__(kTileBlock) k_bounds(const DevMesh m, double* part) {
+__global__ void __launch_bounds__(kTileBlock) k_bounds(int C, const double* ccen,
+                                                       const double* vol, double* part) {
   __shared__ double red[kTileBlock][7];
   double v[7] = {1e300, 1e300, 1e300, -1e300, -1e300, -1e300, 0.0};
-  for (int i = blockIdx.x * kTileBlock + threadIdx.x; i < m.C; i += kBoundsBlocks * kTileBlock) {
+  for (int i = blockIdx.x * kTileBlock + threadIdx.x; i < C; i += kBoundsBlocks * kTileBlock) {
     for (int c = 0; c < 3; c++) {
-      const double x = m.ccen[3 * (size_t)i + c];
+      const double x = ccen[3 * (size_t)i + c];
       v[c] = fmin(v[c], x);
       v[3 + c] = fmax(v[3 + c], x);
     }
-    v[6] += m.vol[i];
+    v[6] += vol[i];
   }
   for (int c = 0; c < 7; c++) red[threadIdx.x][c] = v[c];
   for (int s = kTileBlock / 2; s > 0; s >>= 1) {
@@ -100,16 +101,17 @@ __device__ uint32_t hilbert(uint32_t x[3], int bits) {
   return key;
 }
 
-__global__ void k_hilbert(const DevMesh m, const double* box, int bits, uint32_t* key, int32_t* val) {
+__global__ void k_hilbert(int C, const double* ccen, const int32_t* cell_new, const double* box,
+                          int bits, uint32_t* key, int32_t* val) {
   const double h = box[3];
   const double hi = (double)((1 << bits) - 1);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.C; i += gridDim.x * blockDim.x) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < C; i += gridDim.x * blockDim.x) {
     uint32_t x[3];
     for (int c = 0; c < 3; c++) {
-      const double q = (m.ccen[3 * (size_t)i + c] - box[c]) / h + 0.5;
+      const double q = (ccen[3 * (size_t)i + c] - box[c]) / h + 0.5;
       x[c] = (uint32_t)fmin(fmax(q, 0.0), hi);
     }
-    const int n = m.cell_new[i];
+    const int n = cell_new[i];
     key[n] = hilbert(x, bits);
     val[n] = n;
   }
@@ -381,13 +383,14 @@ inline int pow2_at_least(int n) {
 
 int hilbert_bits() { return 10; }
 
-void launch_cell_curve(const DevMesh& m, const CurveScratch& s, int32_t* order, cudaStream_t st) {
-  const int C = m.C, bits = hilbert_bits();
+void launch_cell_curve(int C, const double* ccen, const double* vol, const int32_t* cell_new,
+                       const CurveScratch& s, int32_t* order, cudaStream_t st) {
+  const int bits = hilbert_bits();
   const int nblk = (C + kSortItems - 1) / kSortItems, n = 256 * nblk;
-  k_bounds<<<kBoundsBlocks, kTileBlock, 0, st>>>(m, s.part);
+  k_bounds<<<kBoundsBlocks, kTileBlock, 0, st>>>(C, ccen, vol, s.part);
   k_box<<<1, 1, 0, st>>>(s.part, C, bits, s.part + 7 * kBoundsBlocks);
-  k_hilbert<<<grid_of(C), kTileBlock, 0, st>>>(m, s.part + 7 * kBoundsBlocks, bits, s.key[0],
-                                               s.val[0]);
+  k_hilbert<<<grid_of(C), kTileBlock, 0, st>>>(C, ccen, cell_new, s.part + 7 * kBoundsBlocks, bits,
+                                               s.key[0], s.val[0]);
   int src = 0;
   for (int shift = 0; shift < 3 * bits; shift += 8, src ^= 1) {
     k_digit_count<<<nblk, kTileBlock, 0, st>>>(s.key[src], C, shift, nblk, s.count);
