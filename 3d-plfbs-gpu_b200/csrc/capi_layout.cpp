@@ -409,6 +409,13 @@ int build_tiles(plfbs_ctx* ctx) {
   t.own = plfbs::march_may_win(false, fp32, tiles, a.F) &&
           plfbs::march_wins(false, fp32, t.n, t.SF, a.F);
   if (!t.own && !(compact && plfbs::march_wins(true, fp32, t.n, t.SF, a.F))) return PLFBS_OK;
+  {
+    KernelArgs b = a;
+    b.tiles = t;
+    int resident = 0;
+    CK(plfbs::prepare_march(b, prec, most_smem, sms, &resident));
+    if (resident < t.n) return PLFBS_OK;
+  }
   const size_t cells = (size_t)t.n * t.SC, faces = (size_t)t.n * t.SF;
   void* p = nullptr;
   TRY(pool_alloc(ctx, &p, 4 * cells));
@@ -438,7 +445,6 @@ int build_tiles(plfbs_ctx* ctx) {
   plfbs::launch_tile_build(a, curve, pos, side, t, got[0], got[1], ctx->stream);
   CK(cudaGetLastError());
   a.tiles = t;
-  CK(plfbs::prepare_march(a, prec, most_smem));
   TRY(pool_alloc(ctx, &p, 4 * (size_t)a.C));
   CK(cudaMemcpyAsync(p, curve, 4 * (size_t)a.C, cudaMemcpyDeviceToDevice, ctx->stream));
   a.red_order = static_cast<const int32_t*>(p);

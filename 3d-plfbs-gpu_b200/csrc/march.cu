@@ -26,6 +26,7 @@
 // and leaves, as do then the others.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
@@ -704,15 +705,24 @@ int march_smem(const KernelArgs& a, int precision, int most, TileArgs& t) {
 
 // The attribute belongs to the kernel on the device, not to a context: threads
 // launch the same instance with tiles of different sizes, so every context sets
-// the same value, the device's limit.
-cudaError_t prepare_march(const KernelArgs& a, int precision, int most) {
+// the same value, the device's limit. `resident`: the blocks that the device holds
+// at once; a cooperative launch of more is refused.
+cudaError_t prepare_march(const KernelArgs& a, int precision, int most, int sms, int* resident) {
   cudaError_t e = cudaSuccess;
   KernelArgs args = a;
+  *resident = 1 << 30;
   for (int k = 0; k < 2 && e == cudaSuccess; k++) {
     e = with_form(args, precision, [&](auto f) {
       using Fm = decltype(f);
-      return cudaFuncSetAttribute(k_march<Fm, march_threads<Fm>()>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+      constexpr int NT = march_threads<Fm>();
+      int per_sm = 0;
+      cudaError_t err = cudaFuncSetAttribute(
+          k_march<Fm, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+      if (err == cudaSuccess)
+        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_march<Fm, NT>, NT,
+                                                            (size_t)a.tiles.smem);
+      *resident = std::min(*resident, per_sm * sms);
+      return err;
     });
     args.compact = 0;  // plfbs_set_layout_compression
   }

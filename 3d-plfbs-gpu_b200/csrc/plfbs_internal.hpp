@@ -409,8 +409,9 @@ void launch_seed(const KernelArgs& a, int precision, bool conserved, cudaStream_
 // up to the step that halts the context. march_smem: a block's dynamic shared
 // memory for t's T, SC and SF within `most` bytes (0: none), and where t's
 // tables go (t.tables, t.place). prepare_march: once per context, before the
-// launches, with a's tiles set and the device's limit on that memory.
-cudaError_t prepare_march(const KernelArgs& a, int precision, int most);
+// launches, with a's tiles set and the device's limit on that memory; *resident
+// returns the blocks that fit on its SMs at once.
+cudaError_t prepare_march(const KernelArgs& a, int precision, int most, int sms, int* resident);
 cudaError_t launch_march(const KernelArgs& a, int precision, int nsteps, cudaStream_t stream);
 int march_max_own();
 int march_max_tiles();
