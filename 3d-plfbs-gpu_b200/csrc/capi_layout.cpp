@@ -364,7 +364,7 @@ int build_tiles(plfbs_ctx* ctx) {
   const int tiles = std::min(sms, plfbs::march_max_tiles());
   plfbs::TileArgs t{};
   t.T = ((a.C + tiles - 1) / tiles + 31) / 32 * 32;
-  if (!coop || t.T > plfbs::march_max_own() || a.F >= (1 << 28) || !ctx->stage.ok)
+  if (!coop || t.T > plfbs::kTileMaxOwn || a.F >= (1 << 28) || !ctx->stage.ok)
     return PLFBS_OK;
   const bool fp32 = prec == PLFBS_FP32_DEVIATION, compact = a.face_rec && a.wtab;
   if (!plfbs::march_may_win(compact, fp32, tiles, a.F)) return PLFBS_OK;

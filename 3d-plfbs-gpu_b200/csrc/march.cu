@@ -38,7 +38,6 @@
 namespace plfbs {
 namespace {
 
-constexpr int kMarchOwn = 1024;  // own cells of a tile, at most
 constexpr int kSpinLimit = 1 << 22;
 
 // Compact tables of up to this many records and weight sets are copied to
@@ -471,7 +470,7 @@ __global__ void __launch_bounds__(NT, 1) k_march(const KernelArgs a, const int n
   using T = typename Fm::T;
   using V = typename Fm::V;
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double red[kMarchOwn / 32][4];
+  __shared__ double red[kTileMaxOwn / 32][4];
   const TileArgs& t = a.tiles;
   constexpr int kRow = row_size<T>();
   T* S = reinterpret_cast<T*>(smem);
@@ -677,8 +676,6 @@ constexpr int march_threads() {
 }
 
 }  // namespace
-
-int march_max_own() { return kMarchOwn; }
 
 int march_max_tiles() { return kMarchTiles; }
 

@@ -18,7 +18,6 @@ namespace {
 
 constexpr int kTileBlock = 256;
 constexpr int kBoundsBlocks = 128;
-constexpr int kTileMaxOwn = 1024;  // own cells of a tile, at most
 constexpr int kSortItems = 4096;  // items per block of the radix sort: 8 warps x 512
 
 // ---------------------------------------------------------------------------
