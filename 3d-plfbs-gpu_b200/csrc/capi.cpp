@@ -329,7 +329,8 @@ bool encode_rows(CUtensorMap* map, const void* base, int cols, long long rows) {
 int check_fault(plfbs_ctx* ctx) {
   if (ctx->stats_host->fault)
     return set_err(ctx, PLFBS_ERR_CUDA,
-                   "a kernel's bounded wait ran out (flux staging); the state is invalid");
+                   "a kernel's bounded wait ran out (flux staging or a march's barrier); the state is "
+                   "invalid");
   return PLFBS_OK;
 }
 
@@ -650,7 +651,7 @@ int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh, const plf
     NvtxRange r("device layout");
     if ((rc = build_device_layout(ctx, *mesh))) return fail(rc);
     // stream-ordered: after the layout kernels that read it
-    if (L.C > plfbs::march_max_tiles() * plfbs::march_max_own()) free_stage(ctx);
+    if (L.C > plfbs::march_max_tiles() * plfbs::kTileMaxOwn) free_stage(ctx);
   }
   {
     NvtxRange r("compact layout");

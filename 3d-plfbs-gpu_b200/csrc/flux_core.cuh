@@ -1,9 +1,10 @@
 // ---------------------------------------------------------------------------
 // Flux core of the FP64 step: the record accesses and the per-face arithmetic
-// that the face kernels (kernels.cu) and the fused stage kernel (stage.cu)
-// share. Every sum and product that a compiler could contract in one kernel
-// and not in another is written as an explicit rounding (fma, __dmul_rn,
-// __dadd_rn), so that all of them compute a face's flux bit for bit alike.
+// that the face kernels (kernels.cu) and the march kernel (march.cu, with its
+// tiles' branch bits in tiles.cu) share. Every sum and product that a compiler
+// could contract in one kernel and not in another is written as an explicit
+// rounding (fma, __dmul_rn, __dadd_rn), so that all of them compute a face's flux
+// bit for bit alike.
 // ---------------------------------------------------------------------------
 #pragma once
 

@@ -1,7 +1,7 @@
 // ---------------------------------------------------------------------------
 // Flux core of the FP32 deviation form (see kernels_fp32.cu for its variables):
 // record accesses and per-face arithmetic shared by the face kernels
-// (kernels_fp32.cu) and the fused stage kernel (stage.cu), with explicit
+// (kernels_fp32.cu) and the march kernel (march.cu, tiles.cu), with explicit
 // roundings as in flux_core.cuh, so that both compute the same bits.
 // ---------------------------------------------------------------------------
 #pragma once
