@@ -651,7 +651,7 @@ int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh, const plf
     NvtxRange r("device layout");
     if ((rc = build_device_layout(ctx, *mesh))) return fail(rc);
     // stream-ordered: after the layout kernels that read it
-    if (L.C > plfbs::march_max_tiles() * plfbs::kTileMaxOwn) free_stage(ctx);
+    if (L.C > plfbs::kMaxTiles * plfbs::kTileMaxOwn) free_stage(ctx);
   }
   {
     NvtxRange r("compact layout");

@@ -361,7 +361,7 @@ int build_tiles(plfbs_ctx* ctx) {
   CK(cudaDeviceGetAttribute(&most_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
   most_smem -= 4096;  // the kernel's own arrays
   ctx->sms = sms;
-  const int tiles = std::min(sms, plfbs::march_max_tiles());
+  const int tiles = std::min(sms, plfbs::kMaxTiles);
   plfbs::TileArgs t{};
   t.T = ((a.C + tiles - 1) / tiles + 31) / 32 * 32;
   if (!coop || t.T > plfbs::kTileMaxOwn || a.F >= (1 << 28) || !ctx->stage.ok)

@@ -22,6 +22,7 @@
 #include "flux_core32.cuh"
 #include "ibm_core.cuh"
 #include "plfbs_internal.hpp"
+#include "residual_core.cuh"
 
 namespace plfbs {
 namespace {
@@ -270,16 +271,7 @@ __global__ void __launch_bounds__(kFinishBlock) k_finish32(const KernelArgs a) {
   __shared__ double red[kFinishBlock / 32][4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double v[4] = {0.0, 0.0, 0.0, 0.0};
-  if (a.red_order) {  // tile by tile, its warps in order
-    const int nw = (a.C + 31) / 32;
-    for (int b = threadIdx.x; b < a.tiles.n; b += kFinishBlock)
-      for (int c = 0; c < 4; c++) {
-        double s = 0.0;
-        for (int w = b * a.red_warps; w < min((b + 1) * a.red_warps, nw); w++)
-          s += a.partial[4 * w + c];
-        v[c] += s;
-      }
-  }
+  if (a.red_order) tile_sums(a, v);
 #pragma unroll 4
   for (int b = threadIdx.x; b < (a.red_order ? 0 : a.nblk_update); b += kFinishBlock) {
     const double2 p0 = __ldg(reinterpret_cast<const double2*>(a.partial + 4LL * b));

@@ -413,13 +413,12 @@ __device__ __forceinline__ bool grid_wait(const unsigned* bar, unsigned target) 
 // The step's norms from the tiles' sums, as k_finish (same order of additions);
 // every block forms them and takes the same decision, block 0 records the
 // step. Returns whether the context halts.
-constexpr int kMarchTiles = 160;  // tiles whose sums one pass covers
 __device__ __forceinline__ bool step_norms(const KernelArgs& a, long long step) {
-  __shared__ double red[kMarchTiles / 32][4];
+  __shared__ double red[kMaxTiles / 32][4];
   __shared__ int stop;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool bad = *(volatile const int*)&a.stats->diverged != 0;
-  if (tid < kMarchTiles) {
+  if (tid < kMaxTiles) {
 #pragma unroll
     for (int c = 0; c < 4; c++) {
       double v = tid < a.tiles.n ? a.partial[4 * tid + c] : 0.0;
@@ -433,7 +432,7 @@ __device__ __forceinline__ bool step_norms(const KernelArgs& a, long long step) 
     double rms = 0.0;
     if (lane < 4) {
       double tot = 0.0;
-      for (int w = 0; w < kMarchTiles / 32; w++) tot += red[w][lane];
+      for (int w = 0; w < kMaxTiles / 32; w++) tot += red[w][lane];
       rms = sqrt(tot / (double)a.C) * (lane == 0 ? a.inv_ref_rho : a.inv_ref_mom);
     }
     const double rho = __shfl_sync(0xffffffffu, rms, 0), u = __shfl_sync(0xffffffffu, rms, 1),
@@ -676,8 +675,6 @@ constexpr int march_threads() {
 }
 
 }  // namespace
-
-int march_max_tiles() { return kMarchTiles; }
 
 // Dynamic shared memory of a block (0: it does not fit in `most`) and the tables
 // that go there beside the rows, in the order of what their loads cost.

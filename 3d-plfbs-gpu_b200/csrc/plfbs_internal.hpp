@@ -299,6 +299,7 @@ struct DevStats {
 //                    is the neighbour), 0xffff in empty slots
 //   count [n]        (local cells, faces)
 constexpr int kTileGhost = 2047;
+constexpr int kMaxTiles = 160;       // tiles of a mesh, at most
 constexpr int kTileMaxOwn = 1024;    // own cells of a tile, at most (k_tile_sort's and k_march's arrays)
 constexpr int kTileMaxCells = 2046;  // local indices fit 11 bits
 constexpr int kTileMaxFaces = 4096;
@@ -414,7 +415,6 @@ void launch_seed(const KernelArgs& a, int precision, bool conserved, cudaStream_
 // returns the blocks that fit on its SMs at once.
 cudaError_t prepare_march(const KernelArgs& a, int precision, int most, int sms, int* resident);
 cudaError_t launch_march(const KernelArgs& a, int precision, int nsteps, cudaStream_t stream);
-int march_max_tiles();
 int march_smem(const KernelArgs& a, int precision, int most, TileArgs& t);
 
 // Exclusive scan of n ints in two levels (layout.cu): item i's prefix is
