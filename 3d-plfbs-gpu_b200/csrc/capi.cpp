@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "capi_internal.hpp"
+#include "device_share.hpp"
 #include "eq_constants.hpp"
 
 using plfbs::DevStats;
@@ -184,34 +185,24 @@ bool marches(const KernelArgs& a) {
          !a.res_debug;
 }
 
-// The SMs that the runs in flight on each device want at once: a march's tiles,
-// or the whole device for a context without. A march holds its SMs for a batch
-// of steps, so marches that fit beside each other run at their own pace (eight
-// of 12 tiles: 3.7 us per step and solve, 8.2 with step graphs), while full
-// ones would take turns (four threads, 32^3 cavity: 40 us per step and solve;
-// 64x32x32 channel 67 FP64, 48 FP32) where the kernels of step graphs fill each
-// other's gaps (27, 52 and 31). So a batch marches if the tiles of all runs in
-// flight fit; the results are the same bits either way.
-constexpr int kWholeDevice = 1 << 12;
-// Steps of a march until the next look at what else is in flight, 15 to 35 ms
-// (its wait and launch cost about 40 us); with a limit on the host's waits a
-// batch is always the full one.
-constexpr int kMarchSteps = 512;
-std::atomic<int> g_sms_wanted[plfbs::kMaxDevices];
+// The SMs a call on a context wants (device_share.hpp): a march's tiles, or all
+// that the kernels over a larger mesh fill. Marches that fit beside each other run
+// at their own pace (eight of 12 tiles: 3.7 us per step and solve, 8.2 with step
+// graphs), while full ones would take turns (four threads, 32^3 cavity: 40 us per
+// step and solve; 64x32x32 channel 67 FP64, 48 FP32) where the kernels of step graphs
+// fill each other's gaps (27, 52 and 31). So a run marches while the SMs that all
+// calls want fit; the results are the same either way.
+int sms_for(const plfbs_ctx* ctx) {
+  return marches(ctx->args) ? ctx->args.tiles.n : sms_for_items(ctx->L.F);
+}
 
-struct InFlight {
-  std::atomic<int>& wanted;
-  const int n;
-  explicit InFlight(const plfbs_ctx* ctx)
-      : wanted(g_sms_wanted[ctx->device >= 0 && ctx->device < plfbs::kMaxDevices ? ctx->device : 0]),
-        n(marches(ctx->args) ? ctx->args.tiles.n : kWholeDevice) {
-    wanted += n;
-  }
-  ~InFlight() { wanted -= n; }
-  InFlight(const InFlight&) = delete;
-  InFlight& operator=(const InFlight&) = delete;
-  bool march_fits(int sms) const { const int w = wanted; return w == n || w <= sms; }
-};
+// Steps per launch of a march, two launches being in flight while the host looks
+// at what else wants the device. Kernels that this library does not know of wait
+// for the end of one (7 to 17 ms) unless the march leaves them an SM; a launch costs
+// about 35 us (64 steps each: 48.8 us per step instead of 48.1 on 65,536 cells FP32).
+constexpr int kMarchSteps = 256;
+// Steps of the graph between two looks, where the context could march.
+constexpr int kGraphSteps = 16;
 
 // One time step: IBM, then 4 x (gradient, flux, update) (Solver_gpu.cu:667-833).
 void enqueue_step(const KernelArgs& a, int prec, cudaStream_t s) {
@@ -336,6 +327,30 @@ int check_fault(plfbs_ctx* ctx) {
 
 
 
+
+// Enqueues the time steps from number `first` on, n of them or fewer, as marches or
+// step graphs. A context that can march looks at the device's other work after each
+// launch, one more being in flight, and stops where it should go on the other way.
+int launch_steps(plfbs_ctx* ctx, const plfbs::DeviceShare& share, bool march, long long first,
+                 long long n) {
+  const bool looks = marches(ctx->args) && ctx->timeout_s == 0;
+  const long long chunk = looks ? (march ? kMarchSteps : kGraphSteps) : n;
+  long long launched = 0;
+  for (int i = 0;; i++) {
+    const long long k = std::min(chunk, n - launched);
+    launched += k;
+    if (march) {
+      CK(plfbs::launch_march(ctx->args, ctx->cfg.precision, first + launched,
+                             looks ? ctx->wanted : nullptr, ctx->sms, ctx->stream));
+    } else {
+      for (long long j = 0; j < k; j++) CK(cudaGraphLaunch(ctx->step_exec, ctx->stream));
+    }
+    if (launched == n) return PLFBS_OK;
+    CK(cudaEventRecord(ctx->look[i & 1], ctx->stream));
+    if (i > 0) CK(cudaEventSynchronize(ctx->look[(i - 1) & 1]));
+    if (share.march_fits(ctx->sms) != march) return PLFBS_OK;
+  }
+}
 
 // Waits at most `seconds` (none if <= 0) for the end of the launched steps
 // (ev1). Running out leaves the context busy: the steps are still in flight
@@ -505,6 +520,8 @@ int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh, const plf
   // first failing index and message); without it, the host threads check
   // them, and their errors are reported before the missing device.
   const bool have_device = check_device(device) == PLFBS_OK;
+  plfbs::DeviceShare share;
+  if (have_device) share.take(device, sms_for_items(mesh->n_faces));
   auto drop = [&](int code, const std::string& m) {
     if (ctx->stream)
       plfbs_destroy(ctx);  // waits for the copies, returns the staged memory
@@ -774,6 +791,8 @@ void plfbs_destroy(plfbs_ctx* ctx) {
   if (ctx->stats_host) give_pinned_stats(ctx->stats_host);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
+  for (cudaEvent_t e : ctx->look)
+    if (e) cudaEventDestroy(e);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
 }
@@ -782,6 +801,7 @@ int plfbs_wall_forces(plfbs_ctx* ctx, const int32_t* wall_bc, int32_t n_wall, do
                       double* cl) {
   NvtxRange range("plfbs_wall_forces");
   TRY(check_ctx(ctx));
+  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
   if (!cd || !cl || n_wall < 0 || (n_wall > 0 && !wall_bc))
     return set_err(ctx, PLFBS_ERR_ARG, "wall_forces needs the wall list and two outputs");
   if (!ctx->have_state) return set_err(ctx, PLFBS_ERR_STATE, "wall_forces before set_state");
@@ -901,6 +921,7 @@ int seed_state(plfbs_ctx* ctx, const double* rho, const double* u, const double*
 int plfbs_set_state(plfbs_ctx* ctx, const double* rho, const double* u, const double* v,
                     const double* w, int64_t n_total) {
   TRY(check_ctx(ctx));
+  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
   const int64_t T = (int64_t)ctx->L.C + ctx->L.B;
   if (!rho || !u || !v || !w || n_total != T)
     return set_err(ctx, PLFBS_ERR_ARG, "set_state needs 4 arrays of n_cells + n_boundary values");
@@ -910,6 +931,7 @@ int plfbs_set_state(plfbs_ctx* ctx, const double* rho, const double* u, const do
 int plfbs_warm_start(plfbs_ctx* ctx, const double* rho, const double* u, const double* v,
                      const double* w, int64_t n_total, const double* node_x, int32_t n_nodes) {
   TRY(check_ctx(ctx));
+  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
   const int64_t T = (int64_t)ctx->L.C + ctx->L.B;
   if (!rho || !u || !v || !w || n_total != T)
     return set_err(ctx, PLFBS_ERR_ARG, "warm_start needs 4 arrays of n_cells + n_boundary values");
@@ -958,6 +980,7 @@ int plfbs_checkpoint_bytes(plfbs_ctx* ctx, int64_t* bytes) {
 int plfbs_save_checkpoint(plfbs_ctx* ctx, void* buf, int64_t bytes) {
   NvtxRange range("plfbs_save_checkpoint");
   TRY(check_ctx(ctx));
+  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
   if (!buf || bytes < checkpoint_size(ctx))
     return set_err(ctx, PLFBS_ERR_ARG, "checkpoint buffer smaller than plfbs_checkpoint_bytes");
   if (!ctx->have_state) return set_err(ctx, PLFBS_ERR_STATE, "checkpoint before set_state");
@@ -1019,6 +1042,7 @@ int plfbs_save_checkpoint(plfbs_ctx* ctx, void* buf, int64_t bytes) {
 int plfbs_load_checkpoint(plfbs_ctx* ctx, const void* buf, int64_t bytes) {
   NvtxRange range("plfbs_load_checkpoint");
   TRY(check_ctx(ctx));
+  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
   if (!buf || bytes < (int64_t)sizeof(CheckpointHeader))
     return set_err(ctx, PLFBS_ERR_ARG, "checkpoint buffer too small");
   CheckpointHeader h;
@@ -1096,21 +1120,15 @@ int plfbs_run(plfbs_ctx* ctx, int64_t max_steps, plfbs_stats* stats, double* his
   float ms_total = 0.f;
   const long long batch = plfbs::kHistoryCap / 2;
   bool halt = ctx->stats_host->halt != 0;
-  const InFlight in_flight(ctx);
+  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
   while (done < max_steps && !halt) {
     NvtxRange r("step batch");
-    const bool march = marches(ctx->args) && in_flight.march_fits(ctx->sms);
-    const long long n = std::min<long long>(
-        march && ctx->timeout_s == 0 ? kMarchSteps : batch, max_steps - done);
+    const bool march = marches(ctx->args) && share.march_fits(ctx->sms);
+    const long long n = std::min<long long>(batch, max_steps - done);
     if (!march && !ctx->step_exec) TRY(build_graph(ctx));
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    if (march) {
-      CK(plfbs::launch_march(ctx->args, ctx->cfg.precision, (int)n, ctx->stream));
-      ctx->grad_stale = ctx->flux_stale = true;  // also where the wait below runs out
-    } else {
-      for (long long k = 0; k < n; k++) CK(cudaGraphLaunch(ctx->step_exec, ctx->stream));
-      ctx->grad_stale = ctx->flux_stale = false;
-    }
+    TRY(launch_steps(ctx, share, march, start + done, n));
+    ctx->grad_stale = ctx->flux_stale = march;  // also where the wait below runs out
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
     TRY(wait_steps(ctx, ctx->timeout_s));
     TRY(read_stats(ctx));
@@ -1204,6 +1222,7 @@ int plfbs_get_state(plfbs_ctx* ctx, double* rho, double* u, double* v, double* w
                     int64_t n_total) {
   NvtxRange range("plfbs_get_state");
   TRY(check_ctx(ctx));
+  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
   const Layout& L = ctx->L;
   const int64_t T = (int64_t)L.C + L.B;
   if (!rho || !u || !v || !w || n_total != T)
@@ -1273,6 +1292,7 @@ int plfbs_set_debug(plfbs_ctx* ctx, int enable) {
 
 int plfbs_run_stages(plfbs_ctx* ctx, int64_t n_stages) {
   TRY(check_ctx(ctx));
+  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
   if (!ctx->have_state) return set_err(ctx, PLFBS_ERR_STATE, "run_stages before set_state");
   if (n_stages > 0) ctx->grad_stale = ctx->flux_stale = false;
   for (int64_t g = 0; g < n_stages; g++) {
@@ -1315,6 +1335,7 @@ static int refresh_introspection(plfbs_ctx* ctx) {
 
 int plfbs_get_gradients(plfbs_ctx* ctx, double* grad, int32_t n_cells) {
   TRY(check_ctx(ctx));
+  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
   const Layout& L = ctx->L;
   if (!grad || n_cells != L.C) return set_err(ctx, PLFBS_ERR_ARG, "gradients: need 12 n_cells");
   TRY(refresh_introspection(ctx));
@@ -1338,6 +1359,7 @@ int plfbs_get_gradients(plfbs_ctx* ctx, double* grad, int32_t n_cells) {
 
 int plfbs_get_face_flux(plfbs_ctx* ctx, double* flux, int32_t n_faces) {
   TRY(check_ctx(ctx));
+  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
   const Layout& L = ctx->L;
   if (!flux || n_faces != L.F) return set_err(ctx, PLFBS_ERR_ARG, "face flux: need 4 n_faces");
   TRY(refresh_introspection(ctx));
@@ -1416,6 +1438,7 @@ int plfbs_get_residual(plfbs_ctx* ctx, double* res, int32_t n_cells) {
 
 int plfbs_profile_steps(plfbs_ctx* ctx, int64_t n_steps, double* ms) {
   TRY(check_ctx(ctx));
+  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
   if (!ms) return set_err(ctx, PLFBS_ERR_ARG, "null output");
   if (!ctx->have_state || ctx->stages_done != 0)
     return set_err(ctx, PLFBS_ERR_STATE, "profile needs a state at a step boundary");
@@ -1462,6 +1485,7 @@ int plfbs_profile_steps(plfbs_ctx* ctx, int64_t n_steps, double* ms) {
 int plfbs_profile_kernels(plfbs_ctx* ctx, int64_t launches, double* ms) {
   NvtxRange range("plfbs_profile_kernels");
   TRY(check_ctx(ctx));
+  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
   if (!ms || launches <= 0) return set_err(ctx, PLFBS_ERR_ARG, "need launches > 0 and an output");
   if (!ctx->have_state || ctx->stages_done != 0)
     return set_err(ctx, PLFBS_ERR_STATE, "profile needs a state at a step boundary");

@@ -7,10 +7,12 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <string>
 #include <vector>
 
+#include "device_share.hpp"
 #include "plfbs.h"
 #include "plfbs_internal.hpp"
 
@@ -22,6 +24,8 @@ struct plfbs_ctx {
   cudaStream_t stream = nullptr;
   cudaGraphExec_t step_exec = nullptr;
   int sms = 0;  // of the device (set for meshes that may march)
+  const int* wanted = nullptr;  // the device's sum of wanted SMs, for kernels (device_share.hpp)
+  cudaEvent_t look[2] = {nullptr, nullptr};  // ends of a march's last two launches
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   plfbs::KernelArgs args{};
   std::vector<void*> allocs;
@@ -125,6 +129,10 @@ int prestage_layout(plfbs_ctx* ctx);
 void release_staging(plfbs_ctx* ctx);
 void free_stage(plfbs_ctx* ctx);
 int build_compact_layout(plfbs_ctx* ctx);
+// SMs that kernels over n items keep busy at most (1,024 items each).
+inline int sms_for_items(long long n) {
+  return (int)std::min<long long>(plfbs::kWholeDevice, std::max(n, 0LL) / 1024 + 1);
+}
 // The tile tables of the march kernel (KernelArgs::tiles; none for a mesh that
 // does not fit one tile per SM).
 int build_tiles(plfbs_ctx* ctx);

@@ -440,11 +440,13 @@ int build_tiles(plfbs_ctx* ctx) {
   t.count = static_cast<int2*>(p);
   TRY(pool_alloc(ctx, &p, (fp32 ? 16 : 32) * ((size_t)a.C + a.B)));
   a.state2 = p;
-  TRY(pool_alloc(ctx, &p, sizeof(unsigned)));
+  TRY(pool_alloc(ctx, &p, 2 * sizeof(unsigned)));
   a.grid_bar = static_cast<unsigned*>(p);
   plfbs::launch_tile_build(a, curve, pos, side, t, got[0], got[1], ctx->stream);
   CK(cudaGetLastError());
   a.tiles = t;
+  ctx->wanted = plfbs::sms_wanted_on_device(ctx->device);
+  for (cudaEvent_t& e : ctx->look) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   TRY(pool_alloc(ctx, &p, 4 * (size_t)a.C));
   CK(cudaMemcpyAsync(p, curve, 4 * (size_t)a.C, cudaMemcpyDeviceToDevice, ctx->stream));
   a.red_order = static_cast<const int32_t*>(p);
@@ -613,6 +615,7 @@ int plfbs_polymesh_geometry(const plfbs_polymesh_view* mesh, double visc, double
   int rc = plfbs::validate_polymesh(*mesh, err);
   if (rc) return set_err(nullptr, rc, err);
   if ((rc = check_device(device))) return rc;
+  const plfbs::DeviceShare share(device, plfbs_capi::sms_for_items(mesh->n_faces));
   // calc_face_delta_t: the cap 3 nu / (gamma fneq_min) (none when fneq_min is 0)
   const double ref_dt = fneq_min != 0 ? visc * 3 / gamma / fneq_min : HUGE_VAL;
   plfbs_ctx tmp;

@@ -28,6 +28,7 @@
 #include <string>
 #include <vector>
 
+#include "device_share.hpp"
 #include "plfbs.h"
 #include "plfbs_gnn.h"
 
@@ -1542,6 +1543,11 @@ int upload_padded(plfbs_gnn* g, float* dst, const float* src, int rows, int cols
   return 0;
 }
 
+// SMs that a pass over the graph keeps busy at most (device_share.hpp).
+int sms_for(const plfbs_gnn* g) {
+  return std::min(plfbs::kWholeDevice, std::max(g->s.n_nodes, g->s.n_edges) / 256 + 1);
+}
+
 int check_g(plfbs_gnn* g) {
   if (!g) return gerr(nullptr, PLFBS_ERR_ARG, "null network");
   GCK(cudaSetDevice(g->device));
@@ -1594,6 +1600,7 @@ int plfbs_gnn_create(const plfbs_gnn_shape* shape, const int32_t* src, const int
     plfbs_gnn_destroy(g);
     return rc;
   };
+  const plfbs::DeviceShare share(device, sms_for(g));
   int rc;
   if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(gerr(g, PLFBS_ERR_CUDA, "stream creation failed"));
@@ -1689,6 +1696,7 @@ int plfbs_gnn_param_count(plfbs_gnn* g, int64_t* n) {
 
 int plfbs_gnn_set_params(plfbs_gnn* g, const float* params, int64_t n) {
   GTRY(check_g(g));
+  const plfbs::DeviceShare share(g->device, sms_for(g));
   if (!params || n != g->P) return gerr(g, PLFBS_ERR_ARG, "parameter count mismatch");
   GCK(cudaMemcpyAsync(g->params, params, n * sizeof(float), cudaMemcpyHostToDevice, g->stream));
   GCK(cudaMemsetAsync(g->adam_m, 0, n * sizeof(float), g->stream));
@@ -1709,6 +1717,7 @@ int plfbs_gnn_get_params(plfbs_gnn* g, float* params, int64_t n) {
 
 int plfbs_gnn_forward(plfbs_gnn* g, const float* node_features, float* y) {
   GTRY(check_g(g));
+  const plfbs::DeviceShare share(g->device, sms_for(g));
   if (!node_features || !y) return gerr(g, PLFBS_ERR_ARG, "null argument");
   GTRY(upload_padded(g, g->feat_n, node_features, g->s.n_nodes, g->s.node_features));
   GTRY(forward(g, false));
@@ -1724,6 +1733,7 @@ int plfbs_gnn_forward(plfbs_gnn* g, const float* node_features, float* y) {
 int plfbs_gnn_gradients(plfbs_gnn* g, const float* node_features, const float* target,
                         double* loss, float* grad) {
   GTRY(check_g(g));
+  const plfbs::DeviceShare share(g->device, sms_for(g));
   if (!node_features || !target || !loss) return gerr(g, PLFBS_ERR_ARG, "null argument");
   GTRY(upload_padded(g, g->feat_n, node_features, g->s.n_nodes, g->s.node_features));
   GTRY(upload_padded(g, g->target, target, g->s.n_nodes, g->s.outputs));
@@ -1738,6 +1748,8 @@ int plfbs_gnn_gradients(plfbs_gnn* g, const float* node_features, const float* t
 
 int plfbs_gnn_train_step(plfbs_gnn* g, const float* node_features, const float* target,
                          float learning_rate, double* loss) {
+  GTRY(check_g(g));
+  const plfbs::DeviceShare share(g->device, sms_for(g));
   GTRY(plfbs_gnn_gradients(g, node_features, target, loss, nullptr));
   g->adam_t++;
   const float c1 = 1.f / (1.f - powf(0.9f, (float)g->adam_t));

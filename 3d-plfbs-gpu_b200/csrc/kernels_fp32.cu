@@ -291,7 +291,8 @@ __global__ void __launch_bounds__(kFinishBlock) k_finish32(const KernelArgs a) {
     double tot[4];
     for (int c = 0; c < 4; c++) {
       tot[c] = 0.0;
-      for (int w = 0; w < kFinishBlock / 32; w++) tot[c] += red[w][c];
+      for (int w = 0; w < (a.red_order ? kMaxTiles / 32 : kFinishBlock / 32); w++)
+        tot[c] += red[w][c];
     }
     DevStats* st = a.stats;
     const double nC = (double)a.C;

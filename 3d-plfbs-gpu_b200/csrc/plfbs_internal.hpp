@@ -390,7 +390,7 @@ struct KernelArgs {
   const int32_t* red_order;
   int red_warps;
   TileArgs tiles;                                 // n = 0: no march kernel
-  unsigned* grid_bar;                             // its barrier counter
+  unsigned* grid_bar;  // its barrier counter, and whether it gives way
 };
 
 // Launchers (kernels.cu; the FP32 deviation form in kernels_fp32.cu). All
@@ -407,14 +407,16 @@ void launch_update(const KernelArgs& a, int precision, int rk, cudaStream_t stre
                    bool finish = true);
 void launch_finish(const KernelArgs& a, int precision, cudaStream_t stream);
 void launch_seed(const KernelArgs& a, int precision, bool conserved, cudaStream_t stream);
-// The march kernel (march.cu): nsteps time steps in one cooperative launch,
-// up to the step that halts the context. march_smem: a block's dynamic shared
-// memory for t's T, SC and SF within `most` bytes (0: none), and where t's
-// tables go (t.tables, t.place). prepare_march: once per context, before the
-// launches, with a's tiles set and the device's limit on that memory; *resident
+// The march kernel (march.cu): the time steps up to number `end` of the run in one
+// cooperative launch, or up to the step that halts the context or, with `wanted`
+// (device_share.hpp), no longer leaves the others their SMs. march_smem: a block's
+// dynamic shared memory for t's T, SC and SF within `most` bytes (0: none), and
+// where t's tables go (t.tables, t.place). prepare_march: once per context, before
+// the launches, with a's tiles set and the device's limit on that memory; *resident
 // returns the blocks that fit on its SMs at once.
 cudaError_t prepare_march(const KernelArgs& a, int precision, int most, int sms, int* resident);
-cudaError_t launch_march(const KernelArgs& a, int precision, int nsteps, cudaStream_t stream);
+cudaError_t launch_march(const KernelArgs& a, int precision, long long end, const int* wanted,
+                         int sms, cudaStream_t stream);
 int march_smem(const KernelArgs& a, int precision, int most, TileArgs& t);
 
 // Exclusive scan of n ints in two levels (layout.cu): item i's prefix is

@@ -204,9 +204,10 @@ int plfbs_polymesh_geometry(const plfbs_polymesh_view* mesh, double visc, double
  * builds the least-squares weights (gradients.cpp:214-313), renumbers for
  * locality, uploads everything to `device` and captures one time step in a
  * CUDA graph. A mesh small enough for its tiles to sit in the SMs' shared
- * memory gets them built instead and marches in one cooperative kernel; while
- * runs of other contexts want its SMs too it takes step graphs, with the same
- * results. The mesh arrays are copied to the device first and checked
+ * memory gets them built instead and marches in cooperative kernels of up to 256
+ * steps; while other calls of this library want its SMs too it takes step graphs,
+ * with the same results. Kernels of the caller's own on the same device may wait
+ * for the end of one such kernel. The mesh arrays are copied to the device first and checked
  * there (the same checks, first failing index and message as on the host
  * threads, which check them when `device` is absent); from page-locked host
  * memory the copies set the pace. The initial state is all zeros until

@@ -275,3 +275,50 @@ def test_march_is_the_stages_with_a_body(plfbs_lib, precision, nodes):
     x = cases.fibonacci_sphere(nodes, 2.0, (8.0, 8.0, 8.0))
     ibm = dict(node_ref=x, stiffness=0.5, radius=2.0, depth=4.0, object_nodes=max(nodes, 2))
     _same_run(ma, c, precision, capi.FLAVOUR_GPU, (True, True), ibm=ibm, exact=nodes == 1)
+
+
+def test_march_gives_way_to_a_network_pass(plfbs_lib):
+    """A march holds its SMs for many steps: it has to stop for another call of the
+    library (a pass waited for the march's launch, some 30 times its own time), and
+    carry on to the same bits."""
+    import time
+
+    from plfbs import gnn
+
+    ma, c = _mesh("box", (64, 32, 32))
+    steps, out = 4000, {}
+
+    def solve(key):
+        s = _solver(ma, c, capi.FP64, capi.FLAVOUR_GPU, 0)
+        s.set_state(_start(ma))
+        _, h = s.run(steps)
+        out[key] = (h, s.gradients(), s.face_flux(), s.get_state())
+        s.close()
+
+    g, _ = _mesh("box", (16, 16, 16))
+    src, dst, ef = gnn.mesh_graph(g)
+    net = gnn.GraphNet(src, dst, ef, g.n_cells, 9, 4, 4)
+    net.set_params(gnn.init_params(9, ef.shape[1], 4, 4, seed=1))
+    x = np.random.default_rng(1).standard_normal((g.n_cells, 9)).astype(np.float32)
+
+    def passes(n):
+        t = []
+        for _ in range(n):
+            t0 = time.perf_counter()
+            y = net.forward(x)
+            t.append(time.perf_counter() - t0)
+        return float(np.median(t)), y
+
+    solve("alone")
+    passes(3)
+    alone, y0 = passes(20)
+    t = threading.Thread(target=solve, args=("beside",))
+    t.start()
+    time.sleep(0.1)
+    beside, y1 = passes(20)
+    t.join()
+    net.close()
+    np.testing.assert_array_equal(y0, y1)
+    for a, b in zip(out["alone"], out["beside"]):
+        np.testing.assert_array_equal(a, b)
+    assert beside < 8 * alone, (alone, beside)
