@@ -328,56 +328,85 @@ int check_fault(plfbs_ctx* ctx) {
 
 
 
-// Enqueues the time steps from number `first` on, n of them or fewer, as marches or
-// step graphs. A context that can march looks at the device's other work after each
-// launch, one more being in flight, and stops where it should go on the other way.
-int launch_steps(plfbs_ctx* ctx, const plfbs::DeviceShare& share, bool march, long long first,
-                 long long n) {
-  const bool looks = marches(ctx->args) && ctx->timeout_s == 0;
-  const long long chunk = looks ? (march ? kMarchSteps : kGraphSteps) : n;
-  long long launched = 0;
-  for (int i = 0;; i++) {
-    const long long k = std::min(chunk, n - launched);
-    launched += k;
-    if (march) {
-      CK(plfbs::launch_march(ctx->args, ctx->cfg.precision, first + launched,
-                             looks ? ctx->wanted : nullptr, ctx->sms, ctx->stream));
-    } else {
-      for (long long j = 0; j < k; j++) CK(cudaGraphLaunch(ctx->step_exec, ctx->stream));
-    }
-    if (launched == n) return PLFBS_OK;
-    CK(cudaEventRecord(ctx->look[i & 1], ctx->stream));
-    if (i > 0) CK(cudaEventSynchronize(ctx->look[(i - 1) & 1]));
-    if (share.march_fits(ctx->sms) != march) return PLFBS_OK;
-  }
-}
+// The end of a host wait of `seconds` from now on (none if <= 0).
+struct Deadline {
+  bool limited;
+  std::chrono::steady_clock::time_point at;
+  explicit Deadline(double seconds)
+      : limited(seconds > 0),
+        at(std::chrono::steady_clock::now() +
+           std::chrono::duration_cast<std::chrono::steady_clock::duration>(
+               std::chrono::duration<double>(limited ? std::min(seconds, 1e9) : 0.0))) {}
+};
 
-// Waits at most `seconds` (none if <= 0) for the end of the launched steps
-// (ev1). Running out leaves the context busy: the steps are still in flight
-// and every call but plfbs_wait and plfbs_destroy returns PLFBS_ERR_TIMEOUT.
-int wait_steps(plfbs_ctx* ctx, double seconds) {
-  if (!(seconds > 0)) {
-    CK(cudaEventSynchronize(ctx->ev1));
-    ctx->busy = false;
+// Waits for the event until the deadline; *ended tells which of them came first.
+int wait_event(plfbs_ctx* ctx, cudaEvent_t ev, const Deadline& deadline, bool* ended) {
+  *ended = true;
+  if (!deadline.limited) {
+    CK(cudaEventSynchronize(ev));
     return PLFBS_OK;
   }
-  const auto deadline = std::chrono::steady_clock::now() + std::chrono::duration<double>(seconds);
   for (;;) {
-    const cudaError_t e = cudaEventQuery(ctx->ev1);
-    if (e == cudaSuccess) {
-      ctx->busy = false;
-      return PLFBS_OK;
-    }
+    const cudaError_t e = cudaEventQuery(ev);
+    if (e == cudaSuccess) return PLFBS_OK;
     if (e != cudaErrorNotReady) CK(e);
-    if (std::chrono::steady_clock::now() >= deadline) {
-      ctx->busy = true;
-      return set_err(ctx, PLFBS_ERR_TIMEOUT,
-                     "the launched steps did not finish within the time limit; they are still "
-                     "in flight (plfbs_wait, then carry on)");
+    if (std::chrono::steady_clock::now() >= deadline.at) {
+      *ended = false;
+      return PLFBS_OK;
     }
     std::this_thread::sleep_for(std::chrono::microseconds(50));
   }
 }
+
+// Enqueues the time steps from number `first` on, n of them or fewer, as marches or
+// step graphs. A context that can march looks at the device's other work after each
+// launch, one more being in flight, and stops where it should go on the other way;
+// from the deadline on it enqueues the rest without a look.
+int launch_steps(plfbs_ctx* ctx, bool march, long long first, long long n,
+                 const Deadline& deadline) {
+  const long long chunk = marches(ctx->args) ? (march ? kMarchSteps : kGraphSteps) : n;
+  long long launched = 0;
+  bool look = true;
+  for (int i = 0;; i++) {
+    const long long k = std::min(chunk, n - launched);
+    launched += k;
+    if (march) {
+      CK(plfbs::launch_march(ctx->args, ctx->cfg.precision, first + launched, ctx->wanted,
+                             ctx->sms, ctx->stream));
+    } else {
+      for (long long j = 0; j < k; j++) CK(cudaGraphLaunch(ctx->step_exec, ctx->stream));
+    }
+    if (launched == n) return PLFBS_OK;
+    if (!look) continue;
+    CK(cudaEventRecord(ctx->look[i & 1], ctx->stream));
+    if (i > 0) TRY(wait_event(ctx, ctx->look[(i - 1) & 1], deadline, &look));
+    if (look && ctx->share.march_fits(ctx->sms) != march) return PLFBS_OK;
+  }
+}
+
+// Waits until the deadline for the end of the launched steps (ev1). Running out
+// leaves the context busy: the steps are still in flight and every call but
+// plfbs_wait and plfbs_destroy returns PLFBS_ERR_TIMEOUT.
+int wait_steps(plfbs_ctx* ctx, const Deadline& deadline) {
+  bool ended = false;
+  TRY(wait_event(ctx, ctx->ev1, deadline, &ended));
+  ctx->busy = !ended;
+  if (!ended)
+    return set_err(ctx, PLFBS_ERR_TIMEOUT,
+                   "the launched steps did not finish within the time limit; they are still "
+                   "in flight (plfbs_wait, then carry on)");
+  return PLFBS_OK;
+}
+
+// The context's share of the device during a run, and after it as long as steps of
+// a run that timed out are in flight.
+struct RunShare {
+  plfbs_ctx* ctx;
+  explicit RunShare(plfbs_ctx* c) : ctx(c) { ctx->share.take(ctx->device, sms_for(ctx)); }
+  ~RunShare() {
+    if (!ctx->busy) ctx->share.drop();
+  }
+};
 
 int check_ctx(plfbs_ctx* ctx) {
   if (!ctx) return set_err(nullptr, PLFBS_ERR_ARG, "null context");
@@ -386,9 +415,10 @@ int check_ctx(plfbs_ctx* ctx) {
     return set_err(ctx, PLFBS_ERR_CUDA, std::string("cudaSetDevice: ") + cudaGetErrorString(e));
   if (ctx->busy) {  // finished since the time-out?
     e = cudaEventQuery(ctx->ev1);
-    if (e == cudaSuccess)
+    if (e == cudaSuccess) {
       ctx->busy = false;
-    else if (e == cudaErrorNotReady)
+      ctx->share.drop();
+    } else if (e == cudaErrorNotReady)
       return set_err(ctx, PLFBS_ERR_TIMEOUT,
                      "steps of a timed-out run are still in flight (plfbs_wait first)");
     else
@@ -1120,17 +1150,18 @@ int plfbs_run(plfbs_ctx* ctx, int64_t max_steps, plfbs_stats* stats, double* his
   float ms_total = 0.f;
   const long long batch = plfbs::kHistoryCap / 2;
   bool halt = ctx->stats_host->halt != 0;
-  const plfbs::DeviceShare share(ctx->device, sms_for(ctx));
+  const RunShare run_share(ctx);
   while (done < max_steps && !halt) {
     NvtxRange r("step batch");
-    const bool march = marches(ctx->args) && share.march_fits(ctx->sms);
+    const bool march = marches(ctx->args) && ctx->share.march_fits(ctx->sms);
     const long long n = std::min<long long>(batch, max_steps - done);
     if (!march && !ctx->step_exec) TRY(build_graph(ctx));
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    TRY(launch_steps(ctx, share, march, start + done, n));
+    const Deadline deadline(ctx->timeout_s);
+    TRY(launch_steps(ctx, march, start + done, n, deadline));
     ctx->grad_stale = ctx->flux_stale = march;  // also where the wait below runs out
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
-    TRY(wait_steps(ctx, ctx->timeout_s));
+    TRY(wait_steps(ctx, deadline));
     TRY(read_stats(ctx));
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
@@ -1189,7 +1220,9 @@ int plfbs_wait(plfbs_ctx* ctx, double seconds) {
   if (e != cudaSuccess)
     return set_err(ctx, PLFBS_ERR_CUDA, std::string("cudaSetDevice: ") + cudaGetErrorString(e));
   if (!ctx->busy) return PLFBS_OK;
-  return wait_steps(ctx, seconds > 0 ? seconds : 1e-9);  // 0: just ask
+  TRY(wait_steps(ctx, Deadline(seconds > 0 ? seconds : 1e-9)));  // 0: just ask
+  ctx->share.drop();
+  return PLFBS_OK;
 }
 
 int plfbs_set_layout_compression(plfbs_ctx* ctx, int32_t on) {

@@ -24,6 +24,7 @@ struct plfbs_ctx {
   cudaStream_t stream = nullptr;
   cudaGraphExec_t step_exec = nullptr;
   int sms = 0;  // of the device (set for meshes that may march)
+  plfbs::DeviceShare share;  // held during a run and while it is busy
   const int* wanted = nullptr;  // the device's sum of wanted SMs, for kernels (device_share.hpp)
   cudaEvent_t look[2] = {nullptr, nullptr};  // ends of a march's last two launches
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;

@@ -322,3 +322,44 @@ def test_march_gives_way_to_a_network_pass(plfbs_lib):
     for a, b in zip(out["alone"], out["beside"]):
         np.testing.assert_array_equal(a, b)
     assert beside < 8 * alone, (alone, beside)
+
+
+def test_timed_out_march_gives_way(plfbs_lib):
+    """Steps of a timed-out run still hold their SMs: another context's run counts
+    them, and they give way to it. Both carry on to the bits of a run alone."""
+    import time
+
+    ma, c = _mesh("box", (64, 32, 32))
+    steps = 2048
+
+    def fresh():
+        s = _solver(ma, c, capi.FP64, capi.FLAVOUR_GPU, 0)
+        s.set_state(_start(ma))
+        s.run(3, history=False)
+        return s
+
+    s = fresh()
+    t0 = time.perf_counter()
+    s.run(steps, history=False)
+    full = time.perf_counter() - t0  # some 140 ms
+    want = s.get_state()
+    s.close()
+    a, b = fresh(), fresh()
+    a.set_timeout(1e-6)
+    with pytest.raises(capi.PlfbsError) as e:
+        a.run(steps, history=False)
+    assert e.value.code == capi.ERR_TIMEOUT
+    t0 = time.perf_counter()
+    b.run(30, history=False)
+    beside = time.perf_counter() - t0
+    assert a.wait(120.0)
+    a.set_timeout(0.0)
+    done = a.run(0, history=False)[0]["steps_done"]
+    assert 3 < done <= steps + 3
+    a.run(steps + 3 - done, history=False)
+    b.run(steps - 30, history=False)
+    np.testing.assert_array_equal(a.get_state(), want)
+    np.testing.assert_array_equal(b.get_state(), want)
+    a.close()
+    b.close()
+    assert beside < full / 3, (beside, full)
