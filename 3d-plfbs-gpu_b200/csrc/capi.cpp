@@ -846,7 +846,6 @@ int plfbs_wall_forces(plfbs_ctx* ctx, const int32_t* wall_bc, int32_t n_wall, do
       return set_err(ctx, PLFBS_ERR_BC, "wall faces need velocity type 1 (Dirichlet) or 2 (Neumann)");
     walls[4 + k] = b;
   }
-  ctx->grad_stale = false;  // the gradients below are the current state's
   // wall_buf: ints [0, 4) zero (a halt flag that reads 0), [4, 4 + n) the
   // walls, then (16-byte aligned) the two sums
   const size_t sums_at = ((size_t)(n_wall + 4) * sizeof(int) + 15) & ~(size_t)15;
@@ -868,6 +867,7 @@ int plfbs_wall_forces(plfbs_ctx* ctx, const int32_t* wall_bc, int32_t n_wall, do
   a.stats = reinterpret_cast<plfbs::DevStats*>(dev_walls);
   plfbs::launch_gradient(a, ctx->cfg.precision, ctx->stream);
   CK(cudaGetLastError());
+  ctx->grad_stale = false;  // they are the current state's
   const double g = ctx->cfg.gamma;
   plfbs::launch_wall_forces(ctx->args, ctx->cfg.precision, dev_walls + 4, n_wall,
                             ctx->cfg.visc * g, g, dev_out, ctx->stream);
@@ -1352,14 +1352,28 @@ static int refresh_introspection(plfbs_ctx* ctx) {
   cudaError_t e = cudaMemsetAsync(zero, 0, sizeof(DevStats), ctx->stream);
   KernelArgs a = ctx->args;
   a.stats = static_cast<DevStats*>(zero);
-  KernelArgs b = a;
-  b.state = a.state2;
-  b.flux_maps = nullptr;
-  plfbs::launch_gradient(b, prec, ctx->stream);
-  if (ctx->flux_stale) plfbs::launch_flux(b, prec, ctx->stream);
-  // a wall-force call since has left the current state's gradients
-  if (!ctx->grad_stale) plfbs::launch_gradient(a, prec, ctx->stream);
-  if (e == cudaSuccess) e = cudaGetLastError();
+  a.state = a.state2;
+  a.flux_maps = nullptr;
+  // a wall-force call since has left gradients of its own: put back behind the fluxes
+  const size_t n = 12 * (size_t)a.C * (prec == PLFBS_FP32_DEVIATION ? sizeof(float) : sizeof(double));
+  void* keep = nullptr;
+  if (!ctx->grad_stale) {
+    const int rc = scratch_alloc(ctx, &keep, n);
+    if (rc) {
+      scratch_free(ctx, zero);
+      return rc;
+    }
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(keep, a.grad, n, cudaMemcpyDeviceToDevice, ctx->stream);
+  }
+  if (e == cudaSuccess) {
+    plfbs::launch_gradient(a, prec, ctx->stream);
+    if (ctx->flux_stale) plfbs::launch_flux(a, prec, ctx->stream);
+    e = cudaGetLastError();
+  }
+  if (keep && e == cudaSuccess)
+    e = cudaMemcpyAsync(a.grad, keep, n, cudaMemcpyDeviceToDevice, ctx->stream);
+  scratch_free(ctx, keep);
   scratch_free(ctx, zero);
   CK(e);
   ctx->grad_stale = ctx->flux_stale = false;

@@ -363,3 +363,29 @@ def test_timed_out_march_gives_way(plfbs_lib):
     a.close()
     b.close()
     assert beside < full / 3, (beside, full)
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.FP32_DEVIATION])
+def test_fluxes_of_a_march_leave_the_wall_forces_gradients(plfbs_lib, precision):
+    """The fluxes of a march are recomputed when asked for, by way of gradients: those
+    that a wall-force call has left since, and the state set after it (its ghosts
+    among it), stay as they were."""
+    ma, c = _mesh("box", (12, 10, 9))
+    q = 0.5 * _start(ma)[::-1].copy()
+    q[:, 3] += 0.5
+    out = []
+    for march in (True, False):
+        s = _solver(ma, c, precision, capi.FLAVOUR_GPU, 0)
+        s.set_state(_start(ma))
+        if march:
+            s.run(STEPS)
+        else:
+            s.run_stages(4 * STEPS)
+        s.wall_forces([0, 1, 2])
+        s.set_state(q)
+        state = s.get_state()
+        out.append((s.face_flux(), s.gradients(), s.get_state()))
+        np.testing.assert_array_equal(out[-1][2], state)
+        s.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
