@@ -486,19 +486,17 @@ __global__ void __launch_bounds__(kFinishBlock) k_finish(const KernelArgs a) {
     if (lane == 0) red[warp][c] = w;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double tot[4];
-    for (int c = 0; c < 4; c++) {
-      tot[c] = 0.0;
-      for (int w = 0; w < (a.red_order ? kMaxTiles / 32 : kFinishBlock / 32); w++)
-        tot[c] += red[w][c];
-    }
+  if (warp > 0) return;
+  double rms = 0.0;  // a lane per component
+  if (lane < 4) {
+    double tot = 0.0;
+    for (int w = 0; w < (a.red_order ? kMaxTiles / 32 : kFinishBlock / 32); w++) tot += red[w][lane];
+    rms = sqrt(tot / (double)a.C) * (lane == 0 ? a.inv_ref_rho : a.inv_ref_mom);
+  }
+  const double rho_rms = __shfl_sync(0xffffffffu, rms, 0), u_rms = __shfl_sync(0xffffffffu, rms, 1),
+               v_rms = __shfl_sync(0xffffffffu, rms, 2), w_rms = __shfl_sync(0xffffffffu, rms, 3);
+  if (lane == 0) {
     DevStats* st = a.stats;
-    const double nC = (double)a.C;
-    const double rho_rms = sqrt(tot[0] / nC) * a.inv_ref_rho;
-    const double u_rms = sqrt(tot[1] / nC) * a.inv_ref_mom;
-    const double v_rms = sqrt(tot[2] / nC) * a.inv_ref_mom;
-    const double w_rms = sqrt(tot[3] / nC) * a.inv_ref_mom;
     const double me = fmax(fmax(w_rms, u_rms), v_rms);  // residuals::max_error
     const long long t = st->steps;
     double* h = st->history[t % kHistoryCap];
