@@ -551,7 +551,6 @@ int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh, const plf
   // them, and their errors are reported before the missing device.
   const bool have_device = check_device(device) == PLFBS_OK;
   plfbs::DeviceShare share;
-  if (have_device) share.take(device, sms_for_items(mesh->n_faces));
   auto drop = [&](int code, const std::string& m) {
     if (ctx->stream)
       plfbs_destroy(ctx);  // waits for the copies, returns the staged memory
@@ -564,6 +563,7 @@ int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh, const plf
     if (cudaSetDevice(device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess)
       return drop(PLFBS_ERR_CUDA, "cudaSetDevice / stream creation failed");
+    share.take(device, sms_for_items(mesh->n_faces));
     if (stage_mesh(ctx, *mesh)) return drop(PLFBS_ERR_CUDA, ctx->err);
   }
   {

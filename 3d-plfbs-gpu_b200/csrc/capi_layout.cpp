@@ -615,7 +615,6 @@ int plfbs_polymesh_geometry(const plfbs_polymesh_view* mesh, double visc, double
   int rc = plfbs::validate_polymesh(*mesh, err);
   if (rc) return set_err(nullptr, rc, err);
   if ((rc = check_device(device))) return rc;
-  const plfbs::DeviceShare share(device, plfbs_capi::sms_for_items(mesh->n_faces));
   // calc_face_delta_t: the cap 3 nu / (gamma fneq_min) (none when fneq_min is 0)
   const double ref_dt = fneq_min != 0 ? visc * 3 / gamma / fneq_min : HUGE_VAL;
   plfbs_ctx tmp;
@@ -623,6 +622,7 @@ int plfbs_polymesh_geometry(const plfbs_polymesh_view* mesh, double visc, double
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&tmp.stream, cudaStreamNonBlocking) != cudaSuccess)
     return set_err(nullptr, PLFBS_ERR_CUDA, "stream creation failed");
+  const plfbs::DeviceShare share(device, plfbs_capi::sms_for_items(mesh->n_faces));
   rc = polymesh_geometry(&tmp, *mesh, ref_dt, *out);
   cudaStreamSynchronize(tmp.stream);  // the scratch frees are stream-ordered
   cudaStreamDestroy(tmp.stream);

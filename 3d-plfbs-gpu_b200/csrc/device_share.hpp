@@ -13,7 +13,8 @@ namespace plfbs {
 
 constexpr int kWholeDevice = 1 << 12;  // more than any device has
 
-// The device's sum, or null past kMaxDevices.
+// The device's sum, or null past kMaxDevices. With the device current: the first
+// call allocates page-locked memory.
 std::atomic<int>* sms_wanted(int device);
 // Where kernels read it (null: not page-locked, host only).
 const int* sms_wanted_on_device(int device);

@@ -1600,10 +1600,10 @@ int plfbs_gnn_create(const plfbs_gnn_shape* shape, const int32_t* src, const int
     plfbs_gnn_destroy(g);
     return rc;
   };
-  const plfbs::DeviceShare share(device, sms_for(g));
   int rc;
   if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(gerr(g, PLFBS_ERR_CUDA, "stream creation failed"));
+  const plfbs::DeviceShare share(device, sms_for(g));
   if ((rc = set_smem<ENC, FP, H>(g)) || (rc = set_smem<EDGE, 3 * H, H>(g)) ||
       (rc = set_smem<NODE, 2 * H, H>(g)) || (rc = set_smem<DEC, H, FP>(g)) ||
       (rc = set_smem_tc<ENC, FP, H>(g)) || (rc = set_smem_tc<EDGE, 3 * H, H>(g)) ||
