@@ -20,10 +20,12 @@
 // by both neighbours, is paid by SMs that were idle.
 //
 // The arithmetic and the order of every sum are those of the three kernels, so
-// a march and the same stages run one by one give the same bits.
+// a march and the same stages run one by one give the same bits (but for the
+// atomic sums of a body's forces in cells that several of its nodes reach).
 //
 // Every wait is bounded: a block that gives up sets the fault and halt flags
-// and leaves, as do then the others.
+// and leaves, as do then the others. Between steps the march gives way to other
+// calls that want its SMs (device_share.hpp).
 #include <cuda_runtime.h>
 
 #include <algorithm>

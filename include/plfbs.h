@@ -207,11 +207,11 @@ int plfbs_polymesh_geometry(const plfbs_polymesh_view* mesh, double visc, double
  * memory gets them built instead and marches in cooperative kernels of up to 256
  * steps; while other calls of this library want its SMs too it takes step graphs,
  * with the same results. Kernels of the caller's own on the same device may wait
- * for the end of one such kernel. The mesh arrays are copied to the device first and checked
- * there (the same checks, first failing index and message as on the host
- * threads, which check them when `device` is absent); from page-locked host
- * memory the copies set the pace. The initial state is all zeros until
- * plfbs_set_state. */
+ * for the end of one such kernel.
+ * The mesh arrays are copied to the device first and checked there (the same
+ * checks, first failing index and message as on the host threads, which check
+ * them when `device` is absent); from page-locked host memory the copies set the
+ * pace. The initial state is all zeros until plfbs_set_state. */
 int plfbs_create(const plfbs_config* cfg, const plfbs_mesh_view* mesh,
                  const plfbs_bc_view* bc, const plfbs_ibm_view* ibm, int device,
                  plfbs_ctx** out);
@@ -291,7 +291,8 @@ int plfbs_get_body_force(plfbs_ctx* ctx, double frontal_area, double* cd, double
 /* Introspection for parity tests (caller numbering). plfbs_run_stages advances
  * by RK stages (4 per time step; the IBM update runs before each step's first
  * stage) with individual kernel launches instead of the step graph or the
- * marching kernel, and gives the same bits. The
+ * marching kernel, and gives the same bits (with a body whose nodes share cells, up to
+ * the order of its atomic sums). The
  * getters return the last stage's interior-cell gradients [12C] (rho, u, v, w,
  * each x, y, z), face fluxes [4F] (x, y, z momentum, mass) and residuals [4C]
  * (u, v, w, rho); residuals are only recorded after plfbs_set_debug(ctx, 1). */
